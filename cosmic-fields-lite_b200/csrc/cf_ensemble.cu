@@ -293,7 +293,7 @@ __global__ void k_counter_add(long long *c, long long v) {
   if (threadIdx.x == 0 && blockIdx.x == 0) *c += v;
 }
 
-// Whole-step tiles of the 7-point ensembles (threads along c x along b, CTAs/SM):
+// Whole-step tiles of the 7-point ensembles (own threads along c x along b, CTAs/SM):
 // shape 0 is cf_rk4_steps' own (FP32 128 x 8 sites, FP64 32 x 8), shape 1 a
 // narrower, taller tile for members whose N is not a multiple of the wide one
 // (FP32 64 x 16, FP64 16 x 16).
@@ -310,7 +310,7 @@ struct EnsStepShape<float, 1> {
 };
 template <>
 struct EnsStepShape<double, 0> {
-  static constexpr int TX = 16, TY = 8, MB = 3;
+  static constexpr int TX = 16, TY = 8, MB = 4;
 };
 template <>
 struct EnsStepShape<double, 1> {
@@ -318,7 +318,12 @@ struct EnsStepShape<double, 1> {
 };
 template <typename S, int SS>
 constexpr size_t ens_step_smem() {
-  return (size_t)StepSmem<S, EnsStepShape<S, SS>::TX, EnsStepShape<S, SS>::TY>::count * sizeof(S);
+  return (size_t)StepSmem<S, EQ_FRW, EnsStepShape<S, SS>::TX, EnsStepShape<S, SS>::TY>::count * sizeof(S);
+}
+// Thread rows of a CTA: the own rows and the tile's ring rows (step_tile).
+template <typename S, int SS>
+constexpr int ens_step_rows() {
+  return EnsStepShape<S, SS>::TY + step_ring_rows(EnsStepShape<S, SS>::TX, EnsStepShape<S, SS>::TY);
 }
 
 // One RK4 step of one work item as cf_rk4_steps' whole-step pass, with the same
@@ -352,11 +357,12 @@ __device__ __forceinline__ void ens_step_item(const EnsArgs &E, const EnsItem &i
   A.dt2 = E.dt / 2.0;
   A.dt = E.dt;
   A.dt6 = E.dt / 6.0;
+  step_coefs_f32(A);
   step_tile<S, EQ_FRW, SH::TX, SH::TY, false>(A, it.c0, it.b0, it.a_begin, it.a_end, sm);
 }
 
 template <typename S, int SS>
-__global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *EnsStepShape<S, SS>::TY, EnsStepShape<S, SS>::MB)
+__global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *ens_step_rows<S, SS>(), EnsStepShape<S, SS>::MB)
     k_ens_step(const EnsArgs E, int step_off) {
   extern __shared__ __align__(16) unsigned char ens_step_sm[];
   ens_step_item<S, SS>(E, E.items[blockIdx.x], *E.step_counter + step_off, step_off,
@@ -370,7 +376,7 @@ __device__ __forceinline__ void ens_xy_back_item(const EnsArgs &E, const EnsItem
   const EnsMember mb = E.members[it.member];
   const int N = mb.N;
   const int c = it.c0 + threadIdx.x * V, b = it.b0 + threadIdx.y;
-  if (threadIdx.x * V >= min(TW, N - it.c0) || b >= N) return;
+  if (threadIdx.x * V >= min(TW, N - it.c0) || threadIdx.y >= EnsStepShape<S, SS>::TY || b >= N) return;
   const long long NN = (long long)N * N;
   for (int a = it.a_begin; a < it.a_end; ++a) {
     const long long site = NN * a + (long long)N * b + c;
@@ -390,7 +396,7 @@ __global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *EnsStepShape<S, SS>::
 // one bounded grid barrier per RK4 step -- every item of step j reads the buffer the
 // items of step j - 1 wrote; a run of odd length ends with phi, pi back in x.
 template <typename S, int SS>
-__global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *EnsStepShape<S, SS>::TY, EnsStepShape<S, SS>::MB)
+__global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *ens_step_rows<S, SS>(), EnsStepShape<S, SS>::MB)
     k_ens_persistent_step(const EnsArgs E) {
   extern __shared__ __align__(16) unsigned char ens_step_sm[];
   __shared__ int next;
@@ -635,7 +641,7 @@ static int launch_persistent(cf_ensemble *E, int nsteps, double dt, cudaStream_t
 template <typename S, int SS>
 static int launch_persistent_step_t(cf_ensemble *E, int nsteps, double dt, cudaStream_t st) {
   auto kern = k_ens_persistent_step<S, SS>;
-  const dim3 block(EnsStepShape<S, SS>::TX, EnsStepShape<S, SS>::TY);
+  const dim3 block(EnsStepShape<S, SS>::TX, ens_step_rows<S, SS>());
   const size_t smem = ens_step_smem<S, SS>();
   if (!E->coop_blocks_step) {
     int per_sm = 0, dev = 0, sms = 0;
@@ -717,7 +723,7 @@ static int launch_items_step(cf_ensemble *E, size_t i0, size_t i1, int step_off,
   A.coef = E->d_coef;
   A.step_counter = E->d_step;
   A.dt = dt;
-  const dim3 block(EnsStepShape<S, SS>::TX, EnsStepShape<S, SS>::TY);
+  const dim3 block(EnsStepShape<S, SS>::TX, BACK ? EnsStepShape<S, SS>::TY : ens_step_rows<S, SS>());
   if constexpr (BACK)
     k_ens_xy_back<S, SS><<<A.n_items, block, 0, st>>>(A);
   else

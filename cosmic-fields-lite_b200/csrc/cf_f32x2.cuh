@@ -43,6 +43,11 @@ template <typename L>
 struct CoefL {
   L hi, lo;
 };
+template <>
+struct CoefL<float2> {
+  float2 hi, lo;
+  __host__ __device__ CoefL<float> lane() const { return CoefL<float>{hi.x, lo.x}; }
+};
 using C2 = CoefL<float2>;
 
 __host__ __device__ inline CoefL<float> coef_f32(double c) {

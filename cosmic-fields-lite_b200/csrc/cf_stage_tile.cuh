@@ -31,6 +31,10 @@ namespace cfb {
 template <typename S, int V>
 struct VecOf;
 template <>
+struct VecOf<double, 1> {
+  using T = double;
+};
+template <>
 struct VecOf<double, 2> {
   using T = double2;
 };
@@ -56,7 +60,9 @@ struct Pack {
 template <typename S, int V>
 __device__ __forceinline__ Pack<S, V> unpack(const typename VecOf<S, V>::T &t) {
   Pack<S, V> r;
-  if constexpr (V == 2) {
+  if constexpr (V == 1) {
+    r.v[0] = t;
+  } else if constexpr (V == 2) {
     r.v[0] = t.x;
     r.v[1] = t.y;
   } else {
@@ -83,7 +89,9 @@ __device__ __forceinline__ Pack<S, V> ldv_rw(const S *p) {
 template <typename S, int V>
 __device__ __forceinline__ void stv(S *p, const Pack<S, V> &r) {
   typename VecOf<S, V>::T t;
-  if constexpr (V == 2) {
+  if constexpr (V == 1) {
+    t = r.v[0];
+  } else if constexpr (V == 2) {
     t.x = r.v[0];
     t.y = r.v[1];
   } else {
@@ -148,6 +156,7 @@ template <>
 struct Coef<float> {
   float hi, lo;
   __host__ __device__ Coef(double c) : hi((float)c), lo((float)(c - (double)(float)c)) {}
+  __host__ __device__ Coef(const CoefL<float> &c) : hi(c.hi), lo(c.lo) {}
   // c v with the product's error random (hi v + lo v); the same operations as c_mul /
   // c_fma of cf_f32x2.cuh
   __device__ __forceinline__ float mul(float v) const { return __fmaf_rn(hi, v, __fmul_rn(lo, v)); }

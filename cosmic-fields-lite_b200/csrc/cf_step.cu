@@ -31,6 +31,7 @@
 
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "cf_internal.cuh"
@@ -374,33 +375,31 @@ static int rk4_steps_pairs_t(cf_ctx *ctx, void *d_state, double t0, double dt, i
 }
 
 // ---- whole-step passes (7-point) -------------------------------------------
-// CTA shape per storage type, measured at N = 512 (ms per step, KG-FRW / comoving
-// step kernel): FP32 32 x 8 threads (128 x 8 sites, 2 CTAs/SM) 1.34 / 2.13 against
-// 16 x 16 1.41 / 2.22 and 16 x 8 (3 CTAs/SM) 1.59 / 2.41; FP64 16 x 8 threads (32 x 8
-// sites, 3 CTAs/SM) 1.71 / 3.14 against 32 x 8 1.85 / 3.19 and 16 x 16 1.81 / 3.32.
+// CTA shape (threads along c and b of the own sites; step_ring_rows more thread rows) and
+// CTAs per SM by storage type and equation, from measurements:
+//   FP32         32 x 8 threads, 128 x 8 sites (the approximate equation 64 x 8), 2 CTAs/SM.
+//                64 x 16 sites: N = 512 FRW 1.05 against 1.06 ms per step, comoving 2.41 against
+//                2.35, N = 200 FRW 0.114 against 0.109.  128 x 16 at 1 CTA/SM: 1.17.
+//   FP64         16 x 8 threads, 32 x 8 sites at 4 CTAs/SM (102 registers): N = 256 FRW 0.192
+//                ms against 0.223 at 3 CTAs/SM; 64 x 8 at 2 CTAs/SM 0.216.  The sqrt
+//                potential, whose root needs more registers, 3 CTAs/SM: 0.266 against 0.338.
+//   FP64 comoving 32 x 8 threads, 64 x 8 sites, 2 CTAs/SM: 32 x 8 sites at 4 / 3 CTAs/SM
+//                within 1% / 10% slower (N = 256).  Fixed Psi (one plane) takes the uncoupled
+//                shape: N = 200 0.145 ms against 0.222, N = 512 2.02 against 2.05.
 template <typename S, int EQ>
 struct StepShape;
-// RW: two ring warps beside the own rows (step_tile RINGW), measured at N = 512
-// (ms per step, step kernel, comoving / KG-FRW): FP32 1.876 / 1.191 against 1.975 /
-// 1.195 without; FP64 2.883 / 1.731 against 2.942 / 1.721; bit-identical.
 template <int EQ>
 struct StepShape<float, EQ> {
   static constexpr int TX = 32, TY = 8, MB = 2;
-  static constexpr bool RW = true;
 };
-// FP64: 32 x 8 sites (57 KB, 3 CTAs per SM), or for the equations with a curvature
-// input 64 x 8 (109 KB, 2 CTAs of 10 warps, at most 102 registers, no spills): N = 512
-// step kernel, comoving 2.81 -> 2.56 ms, KG-FRW 1.69 -> 1.74 (so it keeps 32 x 8);
-// every tile shape forms the same values, so the bits do not change.
 template <int EQ>
 struct StepShape<double, EQ> {
-  static constexpr bool wide = EqOf<EQ>::coupled;
-  static constexpr int TX = wide ? 32 : 16, TY = 8, MB = wide ? 2 : 3;
-  static constexpr bool RW = true;
+  static constexpr bool wide = EqOf<EQ>::coupled && EQ != EQ_FIXED;
+  static constexpr int TX = wide ? 32 : 16, TY = 8, MB = wide ? 2 : (EQ == EQ_SQRT ? 3 : 4);
 };
 template <typename S, int EQ>
 constexpr int step_threads_y() {
-  return StepShape<S, EQ>::TY + (StepShape<S, EQ>::RW ? 2 : 0);
+  return StepShape<S, EQ>::TY + step_ring_rows(StepShape<S, EQ>::TX, StepShape<S, EQ>::TY);
 }
 
 template <typename S, int EQ, bool FULL>
@@ -408,23 +407,37 @@ __global__ void __launch_bounds__(StepShape<S, EQ>::TX *step_threads_y<S, EQ>(),
     k_step(const StepArgs<S> A) {
   extern __shared__ __align__(16) unsigned char step_smem[];
   constexpr int TXs = StepShape<S, EQ>::TX, TYs = StepShape<S, EQ>::TY;
-  using SM = StepSmem<S, TXs, TYs>;
+  using SM = StepSmem<S, EQ, TXs, TYs>;
   const int a_begin = blockIdx.z * A.a_chunk;
-  step_tile<S, EQ, TXs, TYs, FULL, StepShape<S, EQ>::RW>(A, blockIdx.x * SM::TW, blockIdx.y * TYs, a_begin,
-                                                     min(a_begin + A.a_chunk, A.N), reinterpret_cast<S *>(step_smem));
+  step_tile<S, EQ, TXs, TYs, FULL>(A, blockIdx.x * SM::TW, blockIdx.y * TYs, a_begin, min(a_begin + A.a_chunk, A.N),
+                                   reinterpret_cast<S *>(step_smem));
 }
 
-// Planes per CTA: each chunk re-reads 4 halo planes, so chunks are long where the
-// grid stays several waves deep.
-static int step_a_chunk(int N, int tiles_xy) {
-  int chunk = 64;
-  while (chunk > 4 && (long long)tiles_xy * ((N + chunk - 1) / chunk) < 148LL * 6) chunk /= 2;
-  return chunk;
+// Planes per CTA of a whole-step pass with `tiles_xy` tiles and `per_sm` CTAs per SM: equal
+// chunks of at most 72 planes, as many as minimise the time of the waves they make.  A
+// CTA marches over its chunk and `halo` more planes (each chunk forms them again) and
+// starts up in about 1.5 planes' time; with c CTAs on the fullest SM a plane takes 0.27 + c /
+// per_sm of the time it takes per CTA on a full one, and never less than 0.62 (latency; from
+// sweeps of the chunk at N = 48 ... 256, FP64: 0.76 us with one CTA per SM, 1.66 us with
+// four).  Against halving from 64 until the grid is six CTAs per SM deep: N = 128 FP64 39.9
+// -> 33.3 us per step, FP32 13-point 79.8 -> 68.7 us, N = 48 and N = 256 the same chunks.
+static int step_a_chunk(int N, int tiles_xy, int per_sm, int halo) {
+  const double slots = 148.0 * per_sm;
+  int best = 1;
+  double best_cost = 0.0;
+  for (int nc = (N + 71) / 72; nc <= (N + 1) / 2; ++nc) {
+    const int chunk = (N + nc - 1) / nc, chunks = (N + chunk - 1) / chunk;
+    const double n = (double)tiles_xy * chunks, w = std::floor(n / slots), c = std::ceil((n - w * slots) / 148.0);
+    const double last = c > 0 ? std::max(0.62, 0.27 + c / per_sm) : 0.0;  // the wave that is not full
+    const double cost = (chunk + halo + 1.5) * (w * 1.27 + last);
+    if (best_cost == 0.0 || cost < best_cost) best_cost = cost, best = chunk;
+  }
+  return best;
 }
 
 template <typename S, int EQ, bool FULL>
 static int launch_step_k(cf_ctx *ctx, const StepArgs<S> &A, dim3 grid, cudaStream_t st) {
-  using SM = StepSmem<S, StepShape<S, EQ>::TX, StepShape<S, EQ>::TY>;
+  using SM = StepSmem<S, EQ, StepShape<S, EQ>::TX, StepShape<S, EQ>::TY>;
   constexpr size_t bytes = (size_t)SM::count * sizeof(S);
   static unsigned long long attr_set = 0;  // devices on which this instantiation may use > 48 KB
   const unsigned long long bit = 1ull << (ctx->device & 63);
@@ -439,11 +452,12 @@ static int launch_step_k(cf_ctx *ctx, const StepArgs<S> &A, dim3 grid, cudaStrea
 
 template <typename S, int EQ>
 static int launch_step_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
-  using SM = StepSmem<S, StepShape<S, EQ>::TX, StepShape<S, EQ>::TY>;
+  using SM = StepSmem<S, EQ, StepShape<S, EQ>::TX, StepShape<S, EQ>::TY>;
   constexpr int TYs = StepShape<S, EQ>::TY;
   StepArgs<S> A = A0;
   unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, TYs);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy));
+  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4);
+  step_coefs_f32(A);
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
   if (A.N % SM::TW == 0 && A.N % TYs == 0) return launch_step_k<S, EQ, true>(ctx, A, grid, st);
@@ -487,7 +501,7 @@ static int launch_step13_t(cf_ctx *ctx, const StepArgs<float> &A0, cudaStream_t 
   using SM = Step13Smem<S13_TX, S13_TY>;
   StepArgs<float> A = A0;
   const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, S13_TY);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy));
+  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), 1, 8);
   const dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
   if (A.N % SM::TW == 0 && A.N % S13_TY == 0) return launch_step13_k<EQ, true>(ctx, A, grid, st);
