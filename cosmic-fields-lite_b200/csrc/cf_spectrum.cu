@@ -340,29 +340,29 @@ __global__ void k_spec_final(const unsigned long long *bins, const unsigned long
     out[s] = fixed_to_double(bins[2 * s], bins[2 * s + 1], e);
 }
 
-__device__ __forceinline__ long long isqrt_ll(long long s) {
-  long long r = (long long)sqrt((double)s);
-  while (r * r > s) --r;
-  while ((r + 1) * (r + 1) <= s) ++r;
-  return r;
-}
-
-__global__ void k_shells(const unsigned long long *bins, const unsigned long long *maxbits, long long pairs,
-                         const long long *s2counts, double *shells, long long *counts, long long nb, long long ns) {
-  const int e = fixed_exponent(*maxbits, pairs);
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < ns; i += stride) {
-    unsigned long long lo = 0, hi = 0;
-    long long cnt = 0;
-    const long long s_end = min((i + 1) * (i + 1), nb);
-    for (long long s = i * i; s < s_end; ++s) {
-      const unsigned long long l = bins[2 * s];
-      const unsigned long long nl = lo + l;
-      hi += bins[2 * s + 1] + (nl < lo ? 1ull : 0ull);
-      lo = nl;
-      cnt += s2counts[s];
-    }
-    if (shells) shells[i] = fixed_to_double(lo, hi, e);
+// A warp per shell, its lanes the shell's s^2 bins (shell i holds 2i + 1 of them): the
+// 128-bit integer sums do not depend on the order.  (A thread per shell walked them in turn:
+// 276 us at N = 512, 47 us at N = 128.)
+__global__ void __launch_bounds__(256) k_shells(const unsigned long long *bins, const unsigned long long *maxbits,
+                                                long long pairs, const long long *s2counts, double *shells,
+                                                long long *counts, long long nb, long long ns) {
+  const long long i = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (i >= ns) return;
+  const int lane = threadIdx.x & 31;
+  unsigned long long lo = 0, hi = 0;
+  long long cnt = 0;
+  const long long s_end = min((i + 1) * (i + 1), nb);
+  for (long long s = i * i + lane; s < s_end; s += 32) {
+    add128(lo, hi, bins[2 * s], bins[2 * s + 1]);
+    cnt += s2counts[s];
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    const unsigned long long l = __shfl_down_sync(0xffffffffu, lo, o), h = __shfl_down_sync(0xffffffffu, hi, o);
+    add128(lo, hi, l, h);
+    cnt += __shfl_down_sync(0xffffffffu, cnt, o);
+  }
+  if (lane == 0) {
+    if (shells) shells[i] = fixed_to_double(lo, hi, fixed_exponent(*maxbits, pairs));
     if (counts) counts[i] = cnt;
   }
 }
@@ -633,7 +633,7 @@ int density_spectrum_s2(cf_ctx *ctx, const void *d_state, double t, double *d_ou
 
 int s2_to_shells(cf_ctx *ctx, double *d_shells, int64_t *d_counts, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 0));
-  k_shells<<<grid_for(ctx->shells, 128), 128, 0, st>>>(ctx->bins, ctx->maxbits, ctx->spec_mult,
+  k_shells<<<(unsigned)((ctx->shells + 7) / 8), 256, 0, st>>>(ctx->bins, ctx->maxbits, ctx->spec_mult,
                                                        (const long long *)ctx->s2_counts, d_shells,
                                                        (long long *)d_counts, ctx->s2_bins, ctx->shells);
   CF_LAUNCHED(ctx);
