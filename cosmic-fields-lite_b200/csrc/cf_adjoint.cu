@@ -15,11 +15,13 @@
 //   kb1 = h/6 l' + h/2 yb2    ; yb1 = A1^T kb1
 //   l   = l' + yb4 + yb3 + yb2 + yb1
 //   dL/dm += sum_i <kb_i, dA/dm y_i> = sum_i sum_x kb_i.pi(x) (-2 m) y_i.phi(x)
-// The four reverse stages are fused one-pass kernels with the same streaming
-// stencil as the forward stages, the stencil acting on the pi component of kb.
-// The forward stage inputs y_i a reverse step needs (for dL/dm) are recomputed
-// from the nearest checkpoint (every `checkpoint_every` steps): a segment is
-// re-run forward and its states kept, then walked backwards.
+// A reverse step of the 7-point stencil is one pass (cf_adj_tile.cuh) that also forms
+// the forward stage inputs y_i it needs for dL/dm; for the 13-point stencil the four
+// reverse stages are fused one-pass kernels with the same streaming stencil as the
+// forward stages, the stencil acting on the pi component of kb, and the y_i come from
+// the single-stage kernels.  The states come from the nearest checkpoint (every
+// `checkpoint_every` steps): a segment is re-run forward and its states kept (each step
+// from one kept state into the next), then walked backwards.
 //
 // Adjoint variables are FP64 in both precisions; the forward (and its
 // recompute) runs in the context precision, bit-identically.
@@ -27,9 +29,12 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
+#include <utility>
 #include <vector>
 
+#include "cf_adj_tile.cuh"
 #include "cf_internal.cuh"
 
 namespace cfb {
@@ -189,6 +194,28 @@ __global__ void __launch_bounds__(ATX *ATY) k_adj_stage(const AdjArgs<S> A) {
   }
 }
 
+// One whole reverse step (7-point).  32 x 8 sites per CTA, 3 CTAs per SM.
+constexpr int AS_TX = 16, AS_TY = 8, AS_MB = 3;
+template <typename S, bool FULL>
+__global__ void __launch_bounds__(AS_TX *(AS_TY + step_ring_rows(AS_TX, AS_TY)), AS_MB)
+    k_adj_step(const AdjStepArgs<S> A) {
+  extern __shared__ __align__(16) unsigned char adj_smem[];
+  __shared__ double red[AS_TX * (AS_TY + step_ring_rows(AS_TX, AS_TY)) / 32];
+  const int a_begin = blockIdx.z * A.a_chunk, tid = threadIdx.y * AS_TX + threadIdx.x;
+  double dm = adj_tile<S, AS_TX, AS_TY, FULL>(A, blockIdx.x * AS_TX * 2, blockIdx.y * AS_TY, a_begin,
+                                              min(a_begin + A.a_chunk, A.N), adj_smem);
+  // deterministic CTA reduction, then -2m and accumulate into this CTA's slot
+  for (int o = 16; o > 0; o >>= 1) dm += __shfl_down_sync(0xffffffffu, dm, o);
+  if ((tid & 31) == 0) red[tid >> 5] = dm;
+  __syncthreads();
+  if (tid == 0) {
+    double s = 0.0;
+    for (unsigned w = 0; w < blockDim.x * blockDim.y / 32; ++w) s += red[w];
+    const long long cta = ((long long)blockIdx.z * gridDim.y + blockIdx.y) * gridDim.x + blockIdx.x;
+    A.dm_partial[cta] += -A.two_m * s;
+  }
+}
+
 // Adjoint of the energy density rho = 1/2 (pi^2 + m^2 phi^2 + 1/4 inv sum_e (phi_{+e} - phi_{-e})^2):
 //   l.pi  = rb pi,
 //   l.phi = rb m^2 phi + 1/4 inv sum_e [rb_{-e} (phi - phi_{-2e}) - rb_{+e} (phi_{+2e} - phi)],
@@ -311,6 +338,9 @@ __global__ void k_theta_grad(const double *__restrict__ xi, const double *__rest
 // forward stage launcher and step (cf_step.cu)
 int launch_forward_stage(cf_ctx *ctx, int stage, const void *yin, void *yout, void *x, void *xlo, double t,
                          double cy, double dt6, cudaStream_t st);
+// One step from one state into another (cf_step.cu), as rk4_steps takes it in place.
+int rk4_step_to(cf_ctx *ctx, const void *from, void *to, double t0, double dt, int64_t step, cudaStream_t st);
+int step_a_chunk(int N, int tiles_xy, int per_sm, int halo);
 
 }  // namespace cfb
 
@@ -327,8 +357,6 @@ struct cf_adjoint {
   double *dm_partial = nullptr;
   long long dm_slots = 0;
   double dm_direct = 0.0;
-  cufftHandle plan_z2d = 0;
-  bool have_z2d = false;
 };
 
 namespace cfb {
@@ -358,9 +386,42 @@ static int launch_adj_h(cf_adjoint *adj, const AdjArgs<S> &A, cudaStream_t st) {
   return launch_adj<S, 1, STAGE>(adj, A, st);
 }
 
+// Tiles and planes per CTA of the whole reverse step.
+static dim3 adj_step_grid(long long N, int *a_chunk) {
+  const unsigned gx = ceil_div(N, AS_TX * 2), gy = ceil_div(N, AS_TY);
+  *a_chunk = step_a_chunk((int)N, (int)(gx * gy), AS_MB, 4);
+  return dim3(gx, gy, ceil_div(N, *a_chunk));
+}
+
 static long long adj_cta_count(const cf_ctx *ctx) {
   const long long N = ctx->N;
+  if (ctx->p.stencil == 7) {
+    int chunk;
+    const dim3 g = adj_step_grid(N, &chunk);
+    return (long long)g.x * g.y * g.z;
+  }
   return (long long)ceil_div(N, ATX * 2) * (N / ATY) * ceil_div(N, 16);
+}
+
+template <typename S, bool FULL>
+static int launch_adj_step_t(cf_ctx *ctx, const AdjStepArgs<S> &A, dim3 grid, cudaStream_t st) {
+  constexpr size_t bytes = AdjSmem<S, AS_TX, AS_TY>::bytes;
+  static unsigned long long attr_set = 0;  // devices on which this instantiation may use > 48 KB
+  const unsigned long long bit = 1ull << (ctx->device & 63);
+  if (!(attr_set & bit)) {
+    CF_TRY_CUDA(cudaFuncSetAttribute(k_adj_step<S, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    attr_set |= bit;
+  }
+  k_adj_step<S, FULL><<<grid, dim3(AS_TX, AS_TY + step_ring_rows(AS_TX, AS_TY)), bytes, st>>>(A);
+  CF_LAUNCHED(ctx);
+  return CF_OK;
+}
+
+template <typename S>
+static int launch_adj_step(cf_ctx *ctx, AdjStepArgs<S> A, cudaStream_t st) {
+  const dim3 grid = adj_step_grid(A.N, &A.a_chunk);
+  if (A.N % (AS_TX * 2) == 0 && A.N % AS_TY == 0) return launch_adj_step_t<S, true>(ctx, A, grid, st);
+  return launch_adj_step_t<S, false>(ctx, A, grid, st);
 }
 
 int adjoint_create(cf_ctx *ctx, int64_t nsteps, int64_t every, cf_adjoint **out) {
@@ -383,9 +444,10 @@ int adjoint_create(cf_ctx *ctx, int64_t nsteps, int64_t every, cf_adjoint **out)
   bool ok = true;
   a->ckpt.assign(nck, nullptr);
   for (auto &p : a->ckpt) ok = ok && alloc(&p, sb);
-  ok = ok && alloc(&a->seg, sb * (size_t)every) && alloc(&a->Y, 3 * sb);
-  ok = ok && alloc((void **)&a->lam, 2 * fb) && alloc((void **)&a->ka, 2 * fb) && alloc((void **)&a->kb, 2 * fb) &&
-       alloc((void **)&a->accb, 2 * fb) && alloc((void **)&a->rb, fb);
+  ok = ok && alloc(&a->seg, sb * (size_t)every);
+  ok = ok && alloc((void **)&a->lam, 2 * fb) && alloc((void **)&a->ka, 2 * fb) && alloc((void **)&a->rb, fb);
+  if (ctx->p.stencil != 7)  // the single-stage route
+    ok = ok && alloc(&a->Y, 3 * sb) && alloc((void **)&a->kb, 2 * fb) && alloc((void **)&a->accb, 2 * fb);
   a->dm_slots = std::max<long long>(adj_cta_count(ctx), 148 * 16);
   ok = ok && alloc((void **)&a->dm_partial, sizeof(double) * (size_t)a->dm_slots);
   if (!ok) {
@@ -411,7 +473,6 @@ void adjoint_destroy(cf_adjoint *a) {
   cudaFree(a->accb);
   cudaFree(a->rb);
   cudaFree(a->dm_partial);
-  if (a->have_z2d) cufftDestroy(a->plan_z2d);
   delete a;
 }
 
@@ -438,8 +499,8 @@ int adjoint_shell_log_loss(cf_adjoint *a, const void *d_state, const double *h_t
   cf_ctx *ctx = a->ctx;
   const double tT = a->t0 + (double)a->nsteps * a->dt;
   const long long ns = ctx->shells;
-  double *d_sh = nullptr;
-  CF_TRY_CUDA(cudaMallocAsync((void **)&d_sh, sizeof(double) * ns, st));
+  CF_TRY(ensure_small(ctx, (size_t)ns));
+  double *d_sh = ctx->small;
   CF_TRY(density_spectrum_s2(ctx, d_state, tT, nullptr, st));
   CF_TRY(s2_to_shells(ctx, d_sh, nullptr, st));
   std::vector<double> P(ns), g(ns, 0.0);
@@ -461,13 +522,9 @@ int adjoint_shell_log_loss(cf_adjoint *a, const void *d_state, const double *h_t
   const long long pairs = ctx->hc_count / 2;
   k_shell_loss_adjoint<<<gridn(pairs), 256, 0, st>>>(ctx->spec_hc, d_sh, (int)ctx->N, pairs);
   CF_LAUNCHED(ctx);
-  if (!a->have_z2d) {
-    const int N = (int)ctx->N;
-    CF_TRY_CUFFT(cufftPlan3d(&a->plan_z2d, N, N, N, CUFFT_Z2D));
-    a->have_z2d = true;
-  }
-  CF_TRY_CUFFT(cufftSetStream(a->plan_z2d, st));
-  CF_TRY_CUFFT(cufftExecZ2D(a->plan_z2d, (cufftDoubleComplex *)ctx->spec_hc, a->rb));
+  CF_TRY(ensure_z2d(ctx));
+  CF_TRY_CUFFT(cufftSetStream(ctx->plan_z2d1, st));
+  CF_TRY_CUFFT(cufftExecZ2D(ctx->plan_z2d1, (cufftDoubleComplex *)ctx->spec_hc, a->rb));
   // l_T = adjoint of the energy density at t_T
   const double *x = (const double *)d_state;
   if (ctx->p.precision != CF_FP64) {
@@ -481,7 +538,6 @@ int adjoint_shell_log_loss(cf_adjoint *a, const void *d_state, const double *h_t
   CF_LAUNCHED(ctx);
   std::vector<double> part(gb);
   CF_TRY_CUDA(cudaMemcpyAsync(part.data(), a->dm_partial, sizeof(double) * gb, cudaMemcpyDeviceToHost, st));
-  CF_TRY_CUDA(cudaFreeAsync(d_sh, st));
   CF_TRY_CUDA(cudaStreamSynchronize(st));
   double s = 0.0;
   for (double v : part) s += v;
@@ -495,31 +551,51 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
   const long long N3 = ctx->N3;
   const size_t sb = a->state_bytes;
   CF_TRY_CUDA(cudaMemsetAsync(a->dm_partial, 0, sizeof(double) * a->dm_slots, st));
-  S *Y2 = (S *)a->Y;
-  S *Y3 = (S *)((char *)a->Y + sb);
-  S *Y4 = (S *)((char *)a->Y + 2 * sb);
   const double dt = a->dt, dh = dt / 2.0, dt6 = dt / 6.0, dt3 = dt / 3.0;
+  const bool whole = ctx->p.stencil == 7;
+  AdjStepArgs<S> W{};
+  W.N = (int)ctx->N;
+  W.N3 = N3;
+  W.m2 = ctx->p.m * ctx->p.m;
+  W.two_m = 2.0 * ctx->p.m;
+  W.dm_partial = a->dm_partial;
+  W.dt = dt, W.dt2 = dh, W.dt3 = dt3, W.dt6 = dt6;
   AdjArgs<S> A{};
   A.N = (int)ctx->N;
   A.N3 = N3;
-  A.m2 = ctx->p.m * ctx->p.m;
-  A.two_m = 2.0 * ctx->p.m;
+  A.m2 = W.m2;
+  A.two_m = W.two_m;
   A.dm_partial = a->dm_partial;
   A.acc = a->accb;
+  S *Y2 = (S *)a->Y;
+  S *Y3 = (S *)((char *)a->Y + sb);
+  S *Y4 = (S *)((char *)a->Y + 2 * sb);
   const long long nseg = (long long)a->ckpt.size();
   for (long long sgi = nseg - 1; sgi >= 0; --sgi) {
     const int64_t n0 = sgi * a->every;
     const int64_t len = std::min<int64_t>(a->every, a->nsteps - n0);
     char *seg = (char *)a->seg;
-    CF_TRY_CUDA(cudaMemcpyAsync(seg, a->ckpt[sgi], sb, cudaMemcpyDeviceToDevice, st));
-    for (int64_t j = 1; j < len; ++j) {
-      CF_TRY_CUDA(cudaMemcpyAsync(seg + j * sb, seg + (j - 1) * sb, sb, cudaMemcpyDeviceToDevice, st));
-      CF_TRY(rk4_steps(ctx, seg + j * sb, a->t0, dt, n0 + j - 1, 1, st));
-    }
+    // state j of the segment: the checkpoint itself, then the kept states
+    auto state = [&](int64_t j) { return j == 0 ? (char *)a->ckpt[sgi] : seg + j * sb; };
+    for (int64_t j = 1; j < len; ++j) CF_TRY(rk4_step_to(ctx, state(j - 1), state(j), a->t0, dt, n0 + j - 1, st));
     for (int64_t j = len - 1; j >= 0; --j) {
       const int64_t n = n0 + j;
       const double t = a->t0 + (double)n * dt;
-      S *x = (S *)(seg + j * sb);
+      S *x = (S *)state(j);
+      if (whole) {
+        const double ts[3] = {t, t + dh, t + dt};
+        for (int k = 0; k < 3; ++k) {
+          double H;
+          stage_coeffs(ctx->p, ts[k], &W.inv[k], &H);
+          W.hub3[k] = 3.0 * H;
+        }
+        W.lam = a->lam;
+        W.out = a->ka;
+        W.x = x;
+        CF_TRY(launch_adj_step<S>(ctx, W, st));
+        std::swap(a->lam, a->ka);
+        continue;
+      }
       S *xlo = (sizeof(S) == 4) ? x + 2 * N3 : nullptr;
       // recompute the forward stage inputs y2, y3, y4 of step n (bit-identical to the forward)
       CF_TRY(launch_forward_stage(ctx, 1, x, Y2, x, xlo, t, dh, dt6, st));
@@ -594,9 +670,17 @@ int adjoint_set_lambda(cf_adjoint *a, const double *d_lam, double dm_direct, cud
 }
 
 // ---- shell-amplitude parameterisation of the initial field -------------------
-static int ensure_z2d(cf_ctx *ctx, cufftHandle *plan) {
-  const int N = (int)ctx->N;
-  CF_TRY_CUFFT(cufftPlan3d(plan, N, N, N, CUFFT_Z2D));
+int ensure_small(cf_ctx *ctx, size_t doubles) {
+  if (ctx->small_n >= doubles) return CF_OK;
+  cudaFree(ctx->small);  // the calls that used it have returned, and waited for their work
+  ctx->small = nullptr;
+  ctx->small_n = 0;
+  if (cudaMalloc((void **)&ctx->small, doubles * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
+    set_error("cudaMalloc of %zu bytes of scratch failed", doubles * sizeof(double));
+    return CF_ERR_NOMEM;
+  }
+  ctx->small_n = doubles;
   return CF_OK;
 }
 
@@ -605,24 +689,17 @@ int field_from_shell_amplitudes(cf_ctx *ctx, const double *d_xi, const double *d
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
   std::vector<double> sq(ngroups);
   for (int g = 0; g < ngroups; ++g) sq[g] = std::sqrt(h_theta[g]);
-  double *d_sq = nullptr;
-  CF_TRY_CUDA(cudaMallocAsync((void **)&d_sq, sizeof(double) * ngroups, st));
+  CF_TRY(ensure_small(ctx, ngroups));
+  CF_TRY(ensure_z2d(ctx));
+  double *d_sq = ctx->small;
   CF_TRY_CUDA(cudaMemcpyAsync(d_sq, sq.data(), sizeof(double) * ngroups, cudaMemcpyHostToDevice, st));
   const long long pairs = ctx->hc_count / 2;
   k_field_from_theta<<<gridn(pairs), 256, 0, st>>>(d_xi, d_sqrtP, d_sq, spg, ngroups, ctx->spec_hc, (int)ctx->N,
                                                    pairs);
   CF_LAUNCHED(ctx);
-  cufftHandle plan;
-  CF_TRY(ensure_z2d(ctx, &plan));
-  cufftSetStream(plan, st);
-  cufftResult r = cufftExecZ2D(plan, (cufftDoubleComplex *)ctx->spec_hc, d_phi);
-  CF_TRY_CUDA(cudaFreeAsync(d_sq, st));
+  CF_TRY_CUFFT(cufftSetStream(ctx->plan_z2d1, st));
+  CF_TRY_CUFFT(cufftExecZ2D(ctx->plan_z2d1, (cufftDoubleComplex *)ctx->spec_hc, d_phi));
   CF_TRY_CUDA(cudaStreamSynchronize(st));
-  cufftDestroy(plan);
-  if (r != CUFFT_SUCCESS) {
-    set_error("cufftExecZ2D failed (%d)", (int)r);
-    return CF_ERR_CUFFT;
-  }
   return CF_OK;
 }
 
@@ -633,14 +710,13 @@ int shell_amplitude_gradient(cf_ctx *ctx, const double *d_lambda_phi, const doub
   CF_TRY_CUFFT(cufftExecD2Z(ctx->plan_d2z1, (cufftDoubleReal *)d_lambda_phi, (cufftDoubleComplex *)ctx->spec_hc));
   const long long pairs = ctx->hc_count / 2;
   const unsigned blocks = 148 * 4;
-  double *d_part = nullptr;
-  CF_TRY_CUDA(cudaMallocAsync((void **)&d_part, sizeof(double) * blocks * ngroups, st));
+  CF_TRY(ensure_small(ctx, (size_t)blocks * ngroups));
+  double *d_part = ctx->small;
   k_theta_grad<<<blocks, 256, sizeof(double) * 8 * ngroups, st>>>(d_xi, d_sqrtP, ctx->spec_hc, spg, ngroups, d_part,
                                                                   (int)ctx->N, pairs);
   CF_LAUNCHED(ctx);
   std::vector<double> part((size_t)blocks * ngroups);
   CF_TRY_CUDA(cudaMemcpyAsync(part.data(), d_part, sizeof(double) * part.size(), cudaMemcpyDeviceToHost, st));
-  CF_TRY_CUDA(cudaFreeAsync(d_part, st));
   CF_TRY_CUDA(cudaStreamSynchronize(st));
   for (int g = 0; g < ngroups; ++g) {
     double s = 0.0;

@@ -343,7 +343,7 @@ __device__ __forceinline__ void ens_step_item(const EnsArgs &E, const EnsItem &i
   A.xpi = cur + mb.N3;
   A.ophi = nxt;
   A.opi = nxt + mb.N3;
-  A.xlo = (sizeof(S) == 4) ? x + 2 * mb.N3 : nullptr;
+  A.xlo = A.olo = (sizeof(S) == 4) ? x + 2 * mb.N3 : nullptr;
   A.N = mb.N;
   A.N3 = mb.N3;
   A.m2 = mb.m2;

@@ -107,6 +107,14 @@ __global__ void k_scale_by_s2(double *__restrict__ hc, const double *__restrict_
 
 static unsigned blocks_for(long long n) { return (unsigned)std::min<long long>((n + 255) / 256, 148LL * 16); }
 
+int ensure_z2d(cf_ctx *ctx) {
+  if (ctx->have_z2d1) return CF_OK;
+  const int N = (int)ctx->N;
+  CF_TRY_CUFFT(cufftPlan3d(&ctx->plan_z2d1, N, N, N, CUFFT_Z2D));
+  ctx->have_z2d1 = true;
+  return CF_OK;
+}
+
 // The s^2 table on the device (ctx->ic_table), the HC scratch and both plans.
 static int ensure_init(cf_ctx *ctx, const double *h_table, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
@@ -117,11 +125,7 @@ static int ensure_init(cf_ctx *ctx, const double *h_table, cudaStream_t st) {
       return CF_ERR_NOMEM;
     }
   }
-  if (!ctx->have_z2d1) {
-    const int N = (int)ctx->N;
-    CF_TRY_CUFFT(cufftPlan3d(&ctx->plan_z2d1, N, N, N, CUFFT_Z2D));
-    ctx->have_z2d1 = true;
-  }
+  CF_TRY(ensure_z2d(ctx));
   CF_TRY_CUDA(cudaMemcpyAsync(ctx->ic_table, h_table, (size_t)ctx->s2_bins * sizeof(double), cudaMemcpyHostToDevice,
                               st));
   return CF_OK;

@@ -168,6 +168,10 @@ struct cf_ctx {
   cufftHandle plan_z2d1 = 0;
   bool have_z2d1 = false;
   double *ic_table = nullptr;
+  // Small device scratch of calls that return host values (ensure_small): they synchronise
+  // before they return, so no two of them use it at once.
+  double *small = nullptr;
+  size_t small_n = 0;
   unsigned long long *bins = nullptr;   // 2 * s2_bins words: (lo, hi) fixed point
   unsigned long long *maxbits = nullptr;
   long long spec_mult = 0;  // scale multiplier of the last binning (bin_spectrum)
@@ -195,6 +199,9 @@ namespace cfb {
 // Lazily allocated scratch.
 int ensure_rk4_scratch(cf_ctx *ctx);
 int ensure_spectrum_scratch(cf_ctx *ctx, int nfields);
+int ensure_small(cf_ctx *ctx, size_t doubles);
+// The context's FP64 Z2D plan (ctx->plan_z2d1).
+int ensure_z2d(cf_ctx *ctx);
 int ensure_psi(cf_ctx *ctx);
 
 // Returns the cached Psi / dPsi/dt slot for stage time t, refreshing one slot

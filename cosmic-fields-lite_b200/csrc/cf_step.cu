@@ -421,7 +421,7 @@ __global__ void __launch_bounds__(StepShape<S, EQ>::TX *step_threads_y<S, EQ>(),
 // sweeps of the chunk at N = 48 ... 256, FP64: 0.76 us with one CTA per SM, 1.66 us with
 // four).  Against halving from 64 until the grid is six CTAs per SM deep: N = 128 FP64 39.9
 // -> 33.3 us per step, FP32 13-point 79.8 -> 68.7 us, N = 48 and N = 256 the same chunks.
-static int step_a_chunk(int N, int tiles_xy, int per_sm, int halo) {
+int step_a_chunk(int N, int tiles_xy, int per_sm, int halo) {
   const double slots = 148.0 * per_sm;
   int best = 1;
   double best_cost = 0.0;
@@ -545,7 +545,7 @@ static int rk4_steps_fused_t(cf_ctx *ctx, void *d_state, double t0, double dt, i
   A.N3 = N3;
   A.m2 = ctx->p.m * ctx->p.m;
   eq_consts(ctx, &A.q1, &A.q2, &A.cmap, &A.M);
-  A.xlo = (sizeof(S) == 4) ? x + 2 * N3 : nullptr;
+  A.xlo = A.olo = (sizeof(S) == 4) ? x + 2 * N3 : nullptr;
   A.dt2 = dt / 2.0;
   A.dt = dt;
   A.dt6 = dt / 6.0;
@@ -573,6 +573,32 @@ static int rk4_steps_fused_t(cf_ctx *ctx, void *d_state, double t0, double dt, i
   if (pipe) CF_TRY(psi_pipe_end(ctx, st));
   if (cur) CF_TRY_CUDA(cudaMemcpyAsync(x, buf[1], 2 * N3 * sizeof(S), cudaMemcpyDeviceToDevice, st));
   return CF_OK;
+}
+
+// One whole-step pass of an uncoupled equation from one state into another.
+template <typename S>
+static int step_to_t(cf_ctx *ctx, const void *from, void *to, double t, double dt, cudaStream_t st) {
+  const long long N3 = ctx->N3;
+  StepArgs<S> A{};
+  A.N = (int)ctx->N;
+  A.N3 = N3;
+  A.m2 = ctx->p.m * ctx->p.m;
+  eq_consts(ctx, &A.q1, &A.q2, &A.cmap, &A.M);
+  A.xphi = (const S *)from;
+  A.xpi = A.xphi + N3;
+  A.ophi = (S *)to;
+  A.opi = A.ophi + N3;
+  if (sizeof(S) == 4) A.xlo = A.xphi + 2 * N3, A.olo = A.ophi + 2 * N3;
+  A.dt2 = dt / 2.0;
+  A.dt = dt;
+  A.dt6 = dt / 6.0;
+  const double ts[3] = {t, t + dt / 2.0, t + dt};
+  for (int k = 0; k < 3; ++k) {
+    double H;
+    stage_coeffs(ctx->p, ts[k], &A.inv[k], &H);
+    A.hub3[k] = 3.0 * H;
+  }
+  return launch_step<S>(ctx, A, st);
 }
 
 template <typename S>
@@ -706,10 +732,18 @@ int rk4_step_buffers(cf_ctx *ctx, void *d_state, void *acc, void *ya, void *yb, 
   return rk4_step_buffers_t<double>(ctx, d_state, acc, ya, yb, t, dt, st);
 }
 
-int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, int64_t nsteps, cudaStream_t st) {
+// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).
+static bool whole_step_route(const cf_ctx *ctx) {
   const int f = ctx->p.flags;
+  const int shape = shape_of(ctx->p.equation);
   const bool f32 = ctx->p.precision == CF_FP32_COMP;
-  if (f & CF_FLAG_STAGE_KERNELS)
+  const bool coupled = shape == EQ_COMOV || shape == EQ_FIXED || shape == EQ_APPROX;
+  return !(f & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS)) && (ctx->p.stencil == 7 || (f32 && !coupled));
+}
+
+int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, int64_t nsteps, cudaStream_t st) {
+  const bool f32 = ctx->p.precision == CF_FP32_COMP;
+  if (ctx->p.flags & CF_FLAG_STAGE_KERNELS)
     return f32 ? rk4_steps_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
   // 13-point stencil: the whole-step pass for FP32 storage and the equations without
@@ -717,13 +751,24 @@ int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, i
   // equations, where they measured faster (N = 512, FP32_COMP, ms per step: KG-FRW
   // whole-step 2.17 / paired 2.55; comoving 3.86 / 3.81, with an L2 prefetch of the
   // curvature rows 4.45 / 3.81)
-  const int shape = shape_of(ctx->p.equation);
-  const bool coupled = shape == EQ_COMOV || shape == EQ_FIXED || shape == EQ_APPROX;
-  if ((f & CF_FLAG_PAIR_KERNELS) || (ctx->p.stencil != 7 && (!f32 || coupled)))
+  if (!whole_step_route(ctx))
     return f32 ? rk4_steps_pairs_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_pairs_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
   return f32 ? rk4_steps_fused_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
              : rk4_steps_fused_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
+}
+
+// Step `step` of an uncoupled equation from one state into another (the adjoint's kept
+// states): the whole-step pass writes its new state elsewhere anyway; the routes that
+// step in place run on a copy.
+int rk4_step_to(cf_ctx *ctx, const void *from, void *to, double t0, double dt, int64_t step, cudaStream_t st) {
+  const bool f32 = ctx->p.precision == CF_FP32_COMP;
+  if (shape_of(ctx->p.equation) == EQ_FRW && whole_step_route(ctx)) {
+    const double t = t0 + (double)step * dt;
+    return f32 ? step_to_t<float>(ctx, from, to, t, dt, st) : step_to_t<double>(ctx, from, to, t, dt, st);
+  }
+  CF_TRY_CUDA(cudaMemcpyAsync(to, from, 16 * (size_t)ctx->N3, cudaMemcpyDeviceToDevice, st));
+  return rk4_steps(ctx, to, t0, dt, step, 1, st);
 }
 
 int rhs(cf_ctx *ctx, const double *d_x, double *d_dxdt, double t, cudaStream_t st) {

@@ -337,8 +337,8 @@ __device__ __forceinline__ void step13_tile(const StepArgs<float> &A, int c0, in
       comp_update_f32<float2>(xpi, lq, p_add(c1pi, k4), C6, h2, l2);
       *reinterpret_cast<float2 *>(A.ophi + roff + rowoff) = h1;
       *reinterpret_cast<float2 *>(A.opi + roff + rowoff) = h2;
-      *reinterpret_cast<float2 *>(A.xlo + roff + rowoff) = l1;
-      *reinterpret_cast<float2 *>(A.xlo + N3 + roff + rowoff) = l2;
+      *reinterpret_cast<float2 *>(A.olo + roff + rowoff) = l1;
+      *reinterpret_cast<float2 *>(A.olo + N3 + roff + rowoff) = l2;
     }
   }
   cp_async_wait_all();

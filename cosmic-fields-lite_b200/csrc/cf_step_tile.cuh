@@ -82,7 +82,8 @@ struct StepArgs : StepCoefs<S> {
   const S *xpi;
   S *ophi;        // the new phi, pi (another buffer)
   S *opi;
-  S *xlo;         // FP32_COMP lo words [phi | pi], in place
+  const S *xlo;   // FP32_COMP lo words [phi | pi]
+  S *olo;         // the new ones (may be xlo)
   const S *psi[3];   // curvature at t, t + dt/2, t + dt (StageArgs::psi / dpsi)
   const S *dpsi[3];
   const int *cmap;
@@ -541,8 +542,8 @@ __device__ __forceinline__ void step_tile(const StepArgs<S> &A, int c0, int b0, 
           stv(A.ophi + orr, o1v);
           stv(A.opi + orr, o2v);
           if constexpr (sizeof(S) == 4) {
-            stv(A.xlo + orr, o3v);
-            stv(A.xlo + N3 + orr, o4v);
+            stv(A.olo + orr, o3v);
+            stv(A.olo + N3 + orr, o4v);
           }
         }
         Fm = Fq, Wm = Wq;
