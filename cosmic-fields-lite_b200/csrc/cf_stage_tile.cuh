@@ -190,9 +190,9 @@ __device__ __forceinline__ void psi_factors(double e2m1, double &e2, double &e4)
 
 // Laplacian sum (times h^2) at (row, col) of a staged plane whose a-neighbours
 // are q[0..2H] (q[H] the plane itself): 7-point for H = 1, 13-point 4th order for
-// H = 2 (src/fdm3d_cuda.cu:20-83; in FP32 the 13-point sum comes times 12, see
-// lap13_f32).  The single-stage and the paired-stage tiles both form it here, so
-// their sums round identically.
+// H = 2 (src/fdm3d_cuda.cu:20-83; the 13-point sum comes times 12, see lap_coef).
+// The single-stage and the paired-stage tiles both form it here, so their sums round
+// identically.
 template <typename S, int H, int SP, int V, typename T = typename Arith<S>::T>
 __device__ __forceinline__ T lap_at(const Pack<S, V> (&q)[2 * H + 1], const S *sm, int row, int col, int v) {
   const T f0 = (T)q[H].v[v];
@@ -221,7 +221,7 @@ __device__ __forceinline__ T lap_at(const Pack<S, V> (&q)[2 * H + 1], const S *s
                  (T)sm[row * SP + col + 1] + (T)sm[row * SP + col - 1];
     const T s2 = (T)q[4].v[v] + (T)q[0].v[v] + (T)sm[(row + 2) * SP + col] + (T)sm[(row - 2) * SP + col] +
                  (T)sm[row * SP + col + 2] + (T)sm[row * SP + col - 2];
-    return ((T)16 * s1 - s2 - (T)90 * f0) / (T)12;
+    return (T)16 * s1 - s2 - (T)90 * f0;
   }
 }
 
@@ -386,8 +386,8 @@ __device__ __forceinline__ void stage_tile(const StageArgs<S> &A, int c0, int b0
   const S *phi_in = A.yin;
   const S *pi_in = A.yin + N3;
   using T = typename Arith<S>::T;
-  // FP32: the 13-point sum comes times 12 (lap13_f32), its 1/12 rides on the coefficient
-  const double invc = sizeof(T) == 4 ? lap_coef_f32<H>(A.inv) : A.inv;
+  // the 13-point sum comes times 12 (lap_at), its 1/12 rides on the coefficient
+  const double invc = lap_coef<H>(A.inv);
   const StageCoef<T> kc{Coef<T>(A.m2), Coef<T>(invc), Coef<T>(A.hub3), Coef<T>(A.q1), Coef<T>(A.q2)};
   const Coef<T> cy(A.cy), c6(A.dt6);
   const CoarseCols<V> cc = coarse_cols<EQ, V>(A.cmap, act, b, c);

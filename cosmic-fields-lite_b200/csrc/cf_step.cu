@@ -3,9 +3,9 @@
 // One RK4 step (stepper/runge_kutta4_classic.hpp:88-138) is four stages.  By
 // default cf_rk4_steps runs a step as one whole-step pass -- k_step
 // (cf_step_tile.cuh) for the 7-point stencil, k_step13 (cf_step13_tile.cuh) for the
-// 13-point one in FP32 -- and an FP64 13-point step as two paired-stage passes
-// (stages 1+2, 3+4; cf_pair_tile.cuh); all keep the intermediate stage inputs out of
-// HBM and give the same bits.  The four single-stage kernels remain for
+// 13-point one.  The two paired-stage passes (stages 1+2, 3+4; cf_pair_tile.cuh) remain
+// for CF_FLAG_PAIR_KERNELS and the 13-point batched ensembles; all keep the intermediate
+// stage inputs out of HBM and give the same bits.  The four single-stage kernels remain for
 // CF_FLAG_STAGE_KERNELS, the adjoint's recompute, cf_rk4_steps_noalloc and the
 // 13-point persistent ensemble kernel.  A single-stage kernel makes ONE pass over HBM:
 // it streams its stage input y through a 2.5-D blocked stencil and fuses the
@@ -464,60 +464,86 @@ static int launch_step_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
   return launch_step_k<S, EQ, false>(ctx, A, grid, st);
 }
 
-// ---- whole-step passes, 13-point stencil (FP32 storage) -------------------
-// 64 x 16 sites per CTA, two ring warps, 177 KB of shared memory: 1 CTA per SM.  The
-// 2-site ring makes phase 1 form 20 x 68 sites per 1024 own sites (1.33x) against 12 x
-// 68 per 512 (1.59x) at 64 x 8 (108 KB, 2 CTAs per SM): KG-FRW at N = 512 2.165 -> 2.076
-// ms per step.  For the comoving equation, which the paired passes serve (3.54 ms),
-// the whole-step pass measured 3.59 at 64 x 8 and 3.84 at 64 x 16.
-constexpr int S13_TX = 32, S13_TY = 16;
-
-template <int EQ, bool FULL>
-__global__ void __launch_bounds__(S13_TX *(S13_TY + 2), 1) k_step13(const StepArgs<float> A) {
-  extern __shared__ __align__(16) unsigned char step13_smem[];
-  using SM = Step13Smem<S13_TX, S13_TY>;
-  const int a_begin = blockIdx.z * A.a_chunk;
-  step13_tile<EQ, S13_TX, S13_TY, FULL>(A, blockIdx.x * SM::TW, blockIdx.y * S13_TY, a_begin,
-                                        min(a_begin + A.a_chunk, A.N), reinterpret_cast<float *>(step13_smem));
+// ---- whole-step passes, 13-point stencil -----------------------------------
+// CTA shape (own threads along c and b) and CTAs per SM, measured in ms per step against the
+// paired passes (all shapes the same bits):
+//   FP64           16 x 8 threads, 32 x 8 sites, 2 CTAs/SM: N = 256 FRW 0.795 -> 0.368, N = 200
+//                  0.523 -> 0.213, comoving 1.07 -> 0.85.  The sqrt potential needs more
+//                  registers, 32 x 16 sites at 1 CTA/SM: 0.860 -> 0.450 (0.634 at 2).
+//   FP32           8 x 16 threads, 32 x 16 sites, 2 CTAs/SM: N = 512 FRW 1.63 (the earlier whole-step
+//                  pass, which formed ya_phi at every stencil point: 2.14; 64 x 8 sites 1.65).
+//   FP32 coupled   16 x 16 threads, 64 x 16 sites, 1 CTA/SM with 150 registers: N = 512 comoving
+//                  3.53 -> 2.93, fixed Psi at N = 256 0.341 -> 0.274, approximate 0.445 -> 0.411
+//                  (64 x 8 sites at 2 CTAs/SM spills: comoving 4.37).
+template <typename S, int EQ>
+struct Step13Shape;
+template <int EQ>
+struct Step13Shape<float, EQ> {
+  static constexpr bool big = EqOf<EQ>::coupled;
+  static constexpr int TX = big ? 16 : 8, TY = 16, MB = big ? 1 : 2;
+};
+template <int EQ>
+struct Step13Shape<double, EQ> {
+  static constexpr bool big = EQ == EQ_SQRT;
+  static constexpr int TX = 16, TY = big ? 16 : 8, MB = big ? 1 : 2;
+};
+template <typename S, int EQ>
+constexpr int step13_threads_y() {
+  return Step13Shape<S, EQ>::TY + step13_ring_rows(Step13Shape<S, EQ>::TX, Step13Shape<S, EQ>::TY);
 }
 
-template <int EQ, bool FULL>
-static int launch_step13_k(cf_ctx *ctx, const StepArgs<float> &A, dim3 grid, cudaStream_t st) {
-  using SM = Step13Smem<S13_TX, S13_TY>;
-  constexpr size_t bytes = (size_t)SM::count * sizeof(float);
+template <typename S, int EQ, bool FULL>
+__global__ void __launch_bounds__(Step13Shape<S, EQ>::TX *step13_threads_y<S, EQ>(), Step13Shape<S, EQ>::MB)
+    k_step13(const StepArgs<S> A) {
+  extern __shared__ __align__(16) unsigned char step13_smem[];
+  constexpr int TXs = Step13Shape<S, EQ>::TX, TYs = Step13Shape<S, EQ>::TY;
+  using SM = Step13Smem<S, TXs, TYs>;
+  const int a_begin = blockIdx.z * A.a_chunk;
+  step13_tile<S, EQ, TXs, TYs, FULL>(A, blockIdx.x * SM::TW, blockIdx.y * TYs, a_begin, min(a_begin + A.a_chunk, A.N),
+                                     reinterpret_cast<S *>(step13_smem));
+}
+
+template <typename S, int EQ, bool FULL>
+static int launch_step13_k(cf_ctx *ctx, const StepArgs<S> &A, dim3 grid, cudaStream_t st) {
+  using SM = Step13Smem<S, Step13Shape<S, EQ>::TX, Step13Shape<S, EQ>::TY>;
+  constexpr size_t bytes = (size_t)SM::count * sizeof(S);
+  static_assert(bytes <= 227 * 1024, "shared memory of a CTA");
   static unsigned long long attr_set = 0;  // devices on which this instantiation may use > 48 KB
   const unsigned long long bit = 1ull << (ctx->device & 63);
   if (!(attr_set & bit)) {
-    CF_TRY_CUDA(cudaFuncSetAttribute(k_step13<EQ, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    CF_TRY_CUDA(cudaFuncSetAttribute(k_step13<S, EQ, FULL>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
     attr_set |= bit;
   }
-  k_step13<EQ, FULL><<<grid, dim3(S13_TX, S13_TY + 2), bytes, st>>>(A);
+  k_step13<S, EQ, FULL><<<grid, dim3(Step13Shape<S, EQ>::TX, step13_threads_y<S, EQ>()), bytes, st>>>(A);
   CF_LAUNCHED(ctx);
   return CF_OK;
 }
 
-template <int EQ>
-static int launch_step13_t(cf_ctx *ctx, const StepArgs<float> &A0, cudaStream_t st) {
-  using SM = Step13Smem<S13_TX, S13_TY>;
-  StepArgs<float> A = A0;
-  const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, S13_TY);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), 1, 8);
+template <typename S, int EQ>
+static int launch_step13_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
+  using SH = Step13Shape<S, EQ>;
+  using SM = Step13Smem<S, SH::TX, SH::TY>;
+  StepArgs<S> A = A0;
+  const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, SH::TY);
+  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8);
+  for (double &inv : A.inv) inv = lap_coef<2>(inv);  // the 13-point sum's 1/12
+  step_coefs_f32(A);
   const dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
-  if (A.N % SM::TW == 0 && A.N % S13_TY == 0) return launch_step13_k<EQ, true>(ctx, A, grid, st);
-  return launch_step13_k<EQ, false>(ctx, A, grid, st);
+  if (A.N % SM::TW == 0 && A.N % SH::TY == 0) return launch_step13_k<S, EQ, true>(ctx, A, grid, st);
+  return launch_step13_k<S, EQ, false>(ctx, A, grid, st);
 }
 
 template <typename S>
 static int launch_step(cf_ctx *ctx, const StepArgs<S> &A, cudaStream_t st) {
-  if constexpr (sizeof(S) == 4) {
-    if (ctx->p.stencil == 13) {  // the equations without curvature planes (rk4_steps routes the others)
-      switch (shape_of(ctx->p.equation)) {
-        case EQ_LAMBDA: return launch_step13_t<EQ_LAMBDA>(ctx, A, st);
-        case EQ_SQRT: return launch_step13_t<EQ_SQRT>(ctx, A, st);
-        case EQ_FRW: return launch_step13_t<EQ_FRW>(ctx, A, st);
-        default: return set_error("13-point whole-step pass: curvature-coupled equation"), CF_ERR_INVALID;
-      }
+  if (ctx->p.stencil == 13) {
+    switch (shape_of(ctx->p.equation)) {
+      case EQ_COMOV: return launch_step13_t<S, EQ_COMOV>(ctx, A, st);
+      case EQ_LAMBDA: return launch_step13_t<S, EQ_LAMBDA>(ctx, A, st);
+      case EQ_SQRT: return launch_step13_t<S, EQ_SQRT>(ctx, A, st);
+      case EQ_FIXED: return launch_step13_t<S, EQ_FIXED>(ctx, A, st);
+      case EQ_APPROX: return launch_step13_t<S, EQ_APPROX>(ctx, A, st);
+      default: return launch_step13_t<S, EQ_FRW>(ctx, A, st);
     }
   }
   switch (shape_of(ctx->p.equation)) {
@@ -734,11 +760,7 @@ int rk4_step_buffers(cf_ctx *ctx, void *d_state, void *acc, void *ya, void *yb, 
 
 // Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).
 static bool whole_step_route(const cf_ctx *ctx) {
-  const int f = ctx->p.flags;
-  const int shape = shape_of(ctx->p.equation);
-  const bool f32 = ctx->p.precision == CF_FP32_COMP;
-  const bool coupled = shape == EQ_COMOV || shape == EQ_FIXED || shape == EQ_APPROX;
-  return !(f & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS)) && (ctx->p.stencil == 7 || (f32 && !coupled));
+  return !(ctx->p.flags & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS));
 }
 
 int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, int64_t nsteps, cudaStream_t st) {
@@ -746,11 +768,6 @@ int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, i
   if (ctx->p.flags & CF_FLAG_STAGE_KERNELS)
     return f32 ? rk4_steps_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
-  // 13-point stencil: the whole-step pass for FP32 storage and the equations without
-  // curvature planes; the paired passes for FP64 and for the curvature-coupled
-  // equations, where they measured faster (N = 512, FP32_COMP, ms per step: KG-FRW
-  // whole-step 2.17 / paired 2.55; comoving 3.86 / 3.81, with an L2 prefetch of the
-  // curvature rows 4.45 / 3.81)
   if (!whole_step_route(ctx))
     return f32 ? rk4_steps_pairs_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_pairs_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);

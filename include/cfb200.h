@@ -109,9 +109,8 @@ typedef struct cf_params {
 /* cf_rk4_steps runs each step as four single-stage passes instead of the default
  * route; every route gives bit-identical states. */
 #define CF_FLAG_STAGE_KERNELS 2
-/* cf_rk4_steps runs each 7-point step as two paired-stage passes (stages 1+2, 3+4)
- * instead of one whole-step pass (the default for the 7-point stencil; the 13-point
- * stencil always takes the paired passes). */
+/* cf_rk4_steps runs each step as two paired-stage passes (stages 1+2, 3+4)
+ * instead of one whole-step pass (the default for both stencils). */
 #define CF_FLAG_PAIR_KERNELS 4
 /* FP32 storage: the pruned Psi synthesis's last pass (the length-N C2R of every row)
  * runs as the CTA-per-tile kernel instead of the default warp-per-row-group kernel
@@ -210,8 +209,7 @@ int cf_psi_stats(const cf_ctx *ctx, int64_t *refreshes, int64_t *reused);
  * stage times t, t+dt/2, t+dt/2, t+dt (stepper/runge_kutta4_classic.hpp:88-138).
  * Replaces 4 x Equation::operator() + 3 x scale_sum2 + scale_sum5 per step
  * (src/equations_cuda.cu:522-534, :678-731; src/odeint_thrust/thrust_operations.cu:238-313)
- * by one HBM pass per step (7-point stencil; 13-point for the equations without a
- * curvature input) or two (13-point with one); see CF_FLAG_*.  Comoving curvature: the
+ * by one HBM pass per step; see CF_FLAG_*.  Comoving curvature: the
  * next step's Psi slots are synthesised on a side stream of the context, joined by an
  * event on `stream` before the call returns; the host waits only for a pass-A
  * comparison at a step start a few ulp from the previous step's end (CF_FLAG_PSI_NO_REUSE). */
