@@ -302,6 +302,7 @@ int cf_destroy(cf_ctx *ctx) {
   approx_release(ctx);
   if (ctx->have_d2z1) cufftDestroy(ctx->plan_d2z1);
   if (ctx->have_z2d1) cufftDestroy(ctx->plan_z2d1);
+  cudaFree(ctx->fft_tw);
   cudaFree(ctx->small);
   cudaFree(ctx->ic_table);
   if (ctx->have_d2z2) cufftDestroy(ctx->plan_d2z2);

@@ -105,6 +105,7 @@ struct cf_ctx {
   cudaEvent_t psi_fork = nullptr, psi_join = nullptr, psi_stepdone = nullptr;
   cufftHandle plan_psi = 0;  // batched (2) C2R/Z2D into dense N^3
   bool have_plan_psi = false;
+  double2 *fft_tw = nullptr;  // cf_fft3.cuh: e^{2 pi i j / N}, j < N, then e^{2 pi i j / (N/2)}, j < N/2
   // Pruned synthesis when R_fft is exactly zero outside |i|, |j| <= Ka, Kb and
   // k <= Kc (cf_psi.cu): three 1-D passes over the support only.
   bool pruned = false;
@@ -219,6 +220,8 @@ int psi_pipe_fill(cf_ctx *ctx, double t, const double *keep, int nkeep);
 int psi_pipe_use(cf_ctx *ctx, double t, cudaStream_t stream, const void **psi, const void **dpsi);
 int psi_pipe_step_done(cf_ctx *ctx, cudaStream_t stream);
 int psi_pipe_end(cf_ctx *ctx, cudaStream_t stream);
+// The twiddle tables of cf_fft3.cuh (ctx->fft_tw).
+int ensure_fft_tw(cf_ctx *ctx);
 // Psi and dPsi at t, widened to FP64, into d_out (2 N^3 doubles).
 int psi_fields(cf_ctx *ctx, double t, double *d_out, cudaStream_t stream);
 // CF_PSI_* route the next Psi refresh takes.

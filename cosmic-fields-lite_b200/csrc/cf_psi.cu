@@ -27,6 +27,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cf_fft3.cuh"
 #include "cf_internal.cuh"
 
 namespace cfb {
@@ -1253,6 +1254,152 @@ __global__ void k_copy_convert(const double *__restrict__ in, S *__restrict__ ou
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += stride) out[i] = (S)in[i];
 }
 
+// ---- full synthesis, FP64, in three passes of our own (cf_fft3.cuh) -----------
+// Every mode of R_fft may be non-zero (the reference driver's initializer makes it so).  Along
+// a with the transfer factors applied as R is read (once, for both fields), along b in place,
+// along c with e^{2 Psi} - 1 applied as Psi is written: 9 half-complex arrays of traffic
+// against 15 for the transfer kernel, a cuFFT Z2D and the exponential.  Per refresh, ms: N = 256
+// 0.455 -> 0.38, N = 384 2.32 -> 1.35, N = 512 3.87 -> 3.27 (two fields).
+template <int N>
+struct PsiTileA {  // lines along a at one b, L values of k from k0; both fields of it
+  const C64 *R;
+  C64 *out;
+  const C64 *table;  // (T_Psi, T_dPsi) by s^2
+  int k0, b2;
+  long long line;
+  static constexpr int nh = N / 2 + 1;
+  static constexpr long long stride = (long long)N * nh, pairs = stride * N;
+  __device__ __forceinline__ bool in(int l) const { return k0 + l < nh; }
+  __device__ __forceinline__ const C64 *src(int j, int l) const { return R + line + j * stride + l; }
+  __device__ __forceinline__ C64 load(int f, int j, int l, C64 *x) const {
+    const C64 r = *x;
+    if (f) return r;
+    const int as = j <= N / 2 ? j : N - j, k = in(l) ? k0 + l : 0;
+    const C64 t = __ldg(table + (as * as + b2 + k * k));
+    *x = C64{r.x * t.y, r.y * t.y};  // the second field's, for the same thread
+    return C64{r.x * t.x, r.y * t.x};
+  }
+  __device__ __forceinline__ void store(int f, int j, int l, C64 v) const { out[f * pairs + line + j * stride + l] = v; }
+};
+template <int N>
+__global__ void __launch_bounds__(ColShape<N, 2>::T) k_psi_along_a(const C64 *__restrict__ R, C64 *__restrict__ out,
+                                                                  const double *__restrict__ table,
+                                                                  const C64 *__restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char fft_smem[];
+  constexpr int nh = N / 2 + 1, L = ColShape<N, 2>::L, KT = (nh + L - 1) / L;
+  fft_columns<N, 2>(reinterpret_cast<C64 *>(fft_smem), tw, KT * N, [&](int t) {
+    const int b = t / KT, k0 = (t - b * KT) * L, bs = b <= N / 2 ? b : N - b;
+    return PsiTileA<N>{R, out, reinterpret_cast<const C64 *>(table), k0, bs * bs, (long long)b * nh + k0};
+  });
+}
+
+template <int N>
+struct PsiTileB {  // lines along b in one plane a of one field, in place
+  C64 *p;
+  int k0;
+  static constexpr int nh = N / 2 + 1;
+  __device__ __forceinline__ bool in(int l) const { return k0 + l < nh; }
+  __device__ __forceinline__ const C64 *src(int j, int l) const { return p + j * nh + l; }
+  __device__ __forceinline__ C64 load(int, int, int, C64 *x) const { return *x; }
+  __device__ __forceinline__ void store(int, int j, int l, C64 v) const { p[j * nh + l] = v; }
+};
+template <int N>
+__global__ void __launch_bounds__(ColShape<N, 1>::T) k_psi_along_b(C64 *hc, const C64 *__restrict__ tw) {
+  extern __shared__ __align__(16) unsigned char fft_smem[];
+  constexpr int nh = N / 2 + 1, L = ColShape<N, 1>::L, KT = (nh + L - 1) / L;
+  fft_columns<N, 1>(reinterpret_cast<C64 *>(fft_smem), tw, KT * N * 2, [&](int t) {
+    const int fa = t / KT, k0 = (t - fa * KT) * L;  // field and plane
+    return PsiTileB<N>{hc + (long long)fa * N * nh + k0, k0};
+  });
+}
+
+// Rows of both fields, N^2 each, the first field's through e^{2 Psi} - 1.  A length-N C2R of X is an
+// inverse DFT of length M = N/2 of Z[k] = (X[k] + conj X[M-k]) + i (X[k] - conj X[M-k]) w^k,
+// w = e^{2 pi i / N}; X[0] and X[M] enter by their real parts, as in every C2R.
+template <int N>
+struct PsiTileC {
+  const C64 *X, *tw;
+  C64 *out;
+  bool psi;
+  static constexpr int M = N / 2, nh = M + 1;
+  __device__ __forceinline__ const C64 *src() const { return X; }
+  __device__ __forceinline__ C64 load(int j, int r, const C64 *x) const {
+    C64 a = x[r * nh + j], b = x[r * nh + M - j];
+    if (j == 0) a.y = b.y = 0.0;
+    const C64 d = z_mul(C64{a.x - b.x, a.y + b.y}, __ldg(tw + j));
+    return C64{a.x + b.x - d.y, a.y - b.y + d.x};
+  }
+  __device__ __forceinline__ void store(int m, int r, C64 z) const {
+    if (psi) z = C64{e2m1_of(z.x), e2m1_of(z.y)};
+    out[r * M + m] = z;
+  }
+};
+template <int N>
+__global__ void __launch_bounds__(RowShape<N / 2>::T) k_psi_along_c(const C64 *__restrict__ hc, double *__restrict__ out,
+                                                                    const C64 *__restrict__ twN,
+                                                                    const C64 *__restrict__ twM) {
+  extern __shared__ __align__(16) unsigned char fft_smem[];
+  constexpr int M = N / 2, nh = M + 1, ROWS = RowShape<M>::ROWS;
+  static_assert((long long)N * N % ROWS == 0, "whole tiles of one field");
+  fft_rows<M, nh>(reinterpret_cast<C64 *>(fft_smem), twM, 2 * N * N / ROWS, [&](int t) {
+    const long long row0 = (long long)t * ROWS;
+    return PsiTileC<N>{hc + row0 * nh, twN, reinterpret_cast<C64 *>(out) + row0 * M, row0 < (long long)N * N};
+  });
+}
+
+int ensure_fft_tw(cf_ctx *ctx) {
+  if (ctx->fft_tw) return CF_OK;
+  const int N = (int)ctx->N, M = N / 2;
+  std::vector<double2> t((size_t)N + M);
+  const long double two_pi = 6.28318530717958647692528676655900577L;
+  for (int j = 0; j < N; ++j) t[j] = make_double2((double)cosl(two_pi * j / N), (double)sinl(two_pi * j / N));
+  for (int j = 0; j < M; ++j) t[N + j] = t[2 * j];
+  if (cudaMalloc((void **)&ctx->fft_tw, t.size() * sizeof(double2)) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->fft_tw = nullptr;
+    set_error("cudaMalloc twiddle table failed");
+    return CF_ERR_NOMEM;
+  }
+  CF_TRY_CUDA(cudaMemcpy(ctx->fft_tw, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
+  return CF_OK;
+}
+
+template <int N>
+static int full_synthesis_n(cf_ctx *ctx, double *out, cudaStream_t st) {
+  using CA = ColShape<N, 2>;
+  using CB = ColShape<N, 1>;
+  using RS = RowShape<N / 2>;
+  const C64 *tw = ctx->fft_tw;
+  C64 *hc = (C64 *)ctx->psi_hc;
+  const int nh = N / 2 + 1;
+  int ga = 0, gb = 0, gc = 0;
+  CF_TRY_CUDA(fft_grid(k_psi_along_a<N>, CA::T, CA::bytes, ctx->device, (nh + CA::L - 1) / CA::L * N, &ga));
+  CF_TRY_CUDA(fft_grid(k_psi_along_b<N>, CB::T, CB::bytes, ctx->device, (nh + CB::L - 1) / CB::L * N * 2, &gb));
+  CF_TRY_CUDA(fft_grid(k_psi_along_c<N>, RS::T, RS::bytes, ctx->device, 2 * N * N / RS::ROWS, &gc));
+  ProfScope ps(ctx, CF_PROF_PSI_FFT, st);
+  k_psi_along_a<N><<<ga, CA::T, CA::bytes, st>>>((const C64 *)ctx->R_fft, hc, ctx->psi_table, tw);
+  CF_LAUNCHED(ctx);
+  k_psi_along_b<N><<<gb, CB::T, CB::bytes, st>>>(hc, tw);
+  CF_LAUNCHED(ctx);
+  k_psi_along_c<N><<<gc, RS::T, RS::bytes, st>>>(hc, out, tw, tw + N);
+  CF_LAUNCHED(ctx);
+  return CF_OK;
+}
+
+static int full_synthesis(cf_ctx *ctx, void *out, cudaStream_t st) {
+  CF_TRY(ensure_fft_tw(ctx));
+  switch (ctx->N) {
+    case 64: return full_synthesis_n<64>(ctx, (double *)out, st);
+    case 96: return full_synthesis_n<96>(ctx, (double *)out, st);
+    case 128: return full_synthesis_n<128>(ctx, (double *)out, st);
+    case 192: return full_synthesis_n<192>(ctx, (double *)out, st);
+    case 256: return full_synthesis_n<256>(ctx, (double *)out, st);
+    case 384: return full_synthesis_n<384>(ctx, (double *)out, st);
+    case 512: return full_synthesis_n<512>(ctx, (double *)out, st);
+    default: set_error("full synthesis: no passes for N = %lld", (long long)ctx->N); return CF_ERR_INVALID;
+  }
+}
+
 // Slots [slots_alloc, n): 2 N^3 words each and their ready events.
 static int alloc_psi_slots(cf_ctx *ctx, int n) {
   const size_t w = ctx->word;
@@ -1561,6 +1708,9 @@ static int refresh_slot(cf_ctx *ctx, PsiSlot *v, double t, cudaStream_t st, PsiS
       ctx->pa_last_t = t;
       ctx->pa_last_valid = true;
     }
+  } else if (ctx->word == 8 && fft3_has(ctx->N)) {
+    CF_TRY(ensure_psi_hc(ctx));
+    CF_TRY(full_synthesis(ctx, v->psi, st));
   } else {
     CF_TRY(ensure_psi_hc(ctx));
     CF_TRY(ensure_full_plan(ctx));
