@@ -1,0 +1,147 @@
+// cf_energy.cuh -- the energy density of a state, one warp per 64 sites of a row (shared by the
+// single-lattice observers and the ensembles).
+#pragma once
+
+#include "cf_stage_tile.cuh"
+
+namespace cfb {
+
+// ---- energy density -----------------------------------------------------
+// Potential term of the energy density by equation (ED_*):
+//   ED_QUAD    1/2 m^2 phi^2                                (src/equations_cuda.cu:332-369, lambda = 0)
+//   ED_LAMBDA  1/2 m^2 phi^2 + 1/4 lambda phi^4              (:332-369)
+//   ED_SQRT    m^2 f_a^2 (sqrt(1 + phi^2/f_a^2) - 1)         (:431-449)
+//   ED_CURV    1/2 m^2 phi^2 with e^{-2Psi} kinetic and e^{2Psi} gradient weights (:451-473)
+// and rho = 1/2 pi^2 w_k + 1/8 inv w_g sum_axes (phi_{+1} - phi_{-1})^2 + V
+// (src/equations.cpp:38-69, :106-138, :265-322 for the CPU twins).  `psi` holds
+// e^{2 Psi} - 1.  The sqrt potential is formed as m^2 phi^2 / (sqrt(1 + phi^2/f_a^2) + 1),
+// the same value without the cancellation of sqrt(1 + u) - 1 at small u.
+enum EdKind : int { ED_QUAD = 0, ED_LAMBDA = 1, ED_SQRT = 2, ED_CURV = 3 };
+
+// A warp takes 64 sites of a row (two per lane, moved as one vector) and marches along a:
+// phi of planes a - 1, a, a + 1 is read and widened once per plane and kept in registers, the
+// c-neighbours come from the lanes beside, the rows b +- 1 from L1 (a CTA's 8 warps take
+// consecutive b).  No barrier: a warp's loads of a plane are independent of each other and
+// of the other warps.  With a row per block and every stencil point loaded and widened on
+// its own the pass waited on memory at a third of the bandwidth: N = 512 FP32_COMP comoving
+// 1.14 -> 0.84 ms (28 bytes per site: 0.58 at the copy rate).
+// `rowmax` (optional): receives the largest sum of rho^2 over 64 consecutive sites of a row
+// (fixed order, an integer max of the bit pattern): times N^2 ceil(N / 64) it bounds sum_x
+// rho^2, which Parseval turns into a bound on every spectrum bin.
+// MEAN: instead of rho, its mean over a (summed in increasing a, then divided by N) and its
+// slice at a = 0, each optional; one chunk of all planes.
+template <typename S>
+struct EnergyArgs {
+  const S *x, *xlo, *psi;
+  double *rho;
+  double *slice, *mean;
+  int N, a_chunk;
+  double m2, inv, q;
+  unsigned long long *rowmax;
+};
+constexpr int ED_TILE = 64;
+
+template <typename S, int ED, bool MEAN>
+__device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long task, int a0, int a1) {
+  using V2 = typename VecOf<S, 2>::T;
+  const int N = A.N, lane = threadIdx.x & 31;
+  const long long NN = (long long)N * N, N3 = NN * N;
+  const int b = (int)(task % N), c0 = (int)(task / N) * ED_TILE;
+  const int c = c0 + 2 * lane;
+  const bool act = c < N;
+  const int last = min(ED_TILE, N - c0) / 2 - 1;  // the last active lane (N % 8 == 0: not lane 0)
+  const long long row = (long long)N * b + (act ? c : c0);
+  const long long up = (long long)N * (b + 1 == N ? 1 - N : 1), down = (long long)N * (b == 0 ? N - 1 : -1);
+  // the c-neighbour beyond the tile: of lane 0 to the left, of the last lane to the right
+  const long long edge = (long long)N * b + (lane == 0 ? (c0 == 0 ? N - 1 : c0 - 1) : (c + 2 >= N ? 0 : c + 2));
+  const bool at_edge = act && (lane == 0 || lane == last);
+  auto pair = [&](const S *p, const S *lo, long long i) -> double2 {
+    const V2 h = *reinterpret_cast<const V2 *>(p + i);
+    double2 v = make_double2((double)h.x, (double)h.y);
+    if constexpr (sizeof(S) == 4) {
+      const V2 l = *reinterpret_cast<const V2 *>(lo + i);
+      v.x += (double)l.x;
+      v.y += (double)l.y;
+    }
+    return v;
+  };
+  auto one = [&](long long i) -> double {
+    double v = (double)A.x[i];
+    if constexpr (sizeof(S) == 4) v += (double)A.xlo[i];
+    return v;
+  };
+  double2 prev = pair(A.x, A.xlo, NN * (a0 == 0 ? N - 1 : a0 - 1) + row), cur = pair(A.x, A.xlo, NN * a0 + row);
+  const bool vec = (reinterpret_cast<unsigned long long>(A.rho) & 15) == 0;  // a caller's rho may be 8-byte aligned
+  double most = 0.0;
+  double2 sum = make_double2(0.0, 0.0);
+#pragma unroll 2
+  for (int a = a0; a < a1; ++a) {
+    const long long pl = NN * a;
+    const double2 next = pair(A.x, A.xlo, NN * (a + 1 == N ? 0 : a + 1) + row);
+    const double2 n = pair(A.x, A.xlo, pl + row + up), s = pair(A.x, A.xlo, pl + row + down);
+    const double2 p = pair(A.x + N3, A.xlo + N3, pl + row);
+    double e = 0.0;
+    if (at_edge) e = one(pl + edge);
+    double2 g = make_double2(0.0, 0.0);
+    if constexpr (ED == ED_CURV) {
+      const V2 t = *reinterpret_cast<const V2 *>(A.psi + pl + row);
+      g = make_double2((double)t.x, (double)t.y);
+    }
+    double left = __shfl_up_sync(0xffffffffu, cur.y, 1), right = __shfl_down_sync(0xffffffffu, cur.x, 1);
+    if (lane == 0) left = e;
+    if (lane == last) right = e;
+    auto site = [&](double f, double fp, double fm, double fn, double fs, double fr, double fl, double pi, double e2m1) {
+      const double dx = fp - fm, dy = fn - fs, dz = fr - fl;
+      const double grad = dx * dx + dy * dy + dz * dz;
+      if constexpr (ED == ED_CURV) {
+        const double w = 1.0 + e2m1;
+        return 0.5 * (pi * pi / w + A.m2 * f * f + w * 0.25 * A.inv * grad);
+      } else if constexpr (ED == ED_LAMBDA) {
+        return 0.5 * (pi * pi + A.m2 * f * f + 0.25 * A.inv * grad) + 0.25 * A.q * f * f * f * f;
+      } else if constexpr (ED == ED_SQRT) {  // q = 1 / f_a^2
+        return 0.5 * (pi * pi + 0.25 * A.inv * grad) + A.m2 * f * f / (sqrt(1.0 + f * f * A.q) + 1.0);
+      } else {
+        return 0.5 * (pi * pi + A.m2 * f * f + 0.25 * A.inv * grad);
+      }
+    };
+    const double2 r = make_double2(site(cur.x, next.x, prev.x, n.x, s.x, cur.y, left, p.x, g.x),
+                                   site(cur.y, next.y, prev.y, n.y, s.y, right, cur.x, p.y, g.y));
+    if constexpr (MEAN) {
+      if (act && A.slice && a == 0) A.slice[row] = r.x, A.slice[row + 1] = r.y;  // 8-byte aligned
+      sum.x += r.x;
+      sum.y += r.y;
+    } else {
+      if (act) {
+        double *o = A.rho + pl + row;
+        if (vec)
+          *reinterpret_cast<double2 *>(o) = r;
+        else
+          o[0] = r.x, o[1] = r.y;
+      }
+      if (A.rowmax) {
+        double ss = act ? r.x * r.x + r.y * r.y : 0.0;
+        for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
+        most = fmax(most, ss);
+      }
+    }
+    prev = cur, cur = next;
+  }
+  if constexpr (MEAN) {
+    if (act && A.mean) A.mean[row] = sum.x / (double)N, A.mean[row + 1] = sum.y / (double)N;
+  } else {
+    // non-negative doubles order like their bit patterns
+    if (A.rowmax && lane == 0) atomicMax(A.rowmax, (unsigned long long)__double_as_longlong(most));
+  }
+}
+
+// Warp tasks of a lattice, and planes per warp: chunks of at most 32 (two planes more are read
+// per chunk), shorter while `lattices` of them give fewer than 16 warps per SM.
+inline long long energy_tasks(int N) { return (long long)N * ((N + ED_TILE - 1) / ED_TILE); }
+
+inline int energy_chunk(int N, int lattices) {
+  int ch = 32;
+  while (ch > 2 && lattices * energy_tasks(N) * ((N + ch - 1) / ch) < 148LL * 16) ch /= 2;
+  return ch;
+}
+
+}  // namespace cfb

@@ -37,6 +37,7 @@
 #include <map>
 #include <vector>
 
+#include "cf_energy.cuh"
 #include "cf_internal.cuh"
 #include "cf_pair_tile.cuh"
 #include "cf_stage_tile.cuh"
@@ -425,26 +426,19 @@ __global__ void __launch_bounds__(EnsStepShape<S, SS>::TX *ens_step_rows<S, SS>(
   }
 }
 
-// Batched energy density of the members of one size class (blockIdx.y = member in class).
+// Batched energy density of the members of one size class (blockIdx.z = member in class): the
+// march of cf_energy.cuh, rho of the class consecutive.
 template <typename S>
-__global__ void k_ens_energy(const EnsMember *members, const int *class_members, double *rho, int N, double a2) {
-  const EnsMember mb = members[class_members[blockIdx.y]];
-  const long long N3 = mb.N3, NN = (long long)N * N;
+__global__ void __launch_bounds__(256) k_ens_energy(const EnsMember *members, const int *class_members, double *rho,
+                                                    int N, int a_chunk, double a2) {
+  const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (task >= (long long)N * ((N + ED_TILE - 1) / ED_TILE)) return;  // whole warps
+  const EnsMember mb = members[class_members[blockIdx.z]];
   const S *x = (const S *)mb.x;
-  const S *xlo = (sizeof(S) == 4) ? x + 2 * N3 : nullptr;
-  double *out = rho + (long long)blockIdx.y * N3;
-  const double inv = mb.inv_scale / a2;
-  auto phi = [&](long long i) -> double { return (double)x[i] + (xlo ? (double)xlo[i] : 0.0); };
-  const long long stride = (long long)gridDim.x * blockDim.x;
-  for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < N3; i += stride) {
-    const int c = (int)(i % N), b = (int)((i / N) % N), a = (int)(i / NN);
-    const double dx = phi(NN * ((a + 1) % N) + (long long)N * b + c) - phi(NN * ((a + N - 1) % N) + (long long)N * b + c);
-    const double dy = phi(NN * a + (long long)N * ((b + 1) % N) + c) - phi(NN * a + (long long)N * ((b + N - 1) % N) + c);
-    const double dz = phi(NN * a + (long long)N * b + (c + 1) % N) - phi(NN * a + (long long)N * b + (c + N - 1) % N);
-    const double f = phi(i);
-    const double p = (double)x[N3 + i] + (xlo ? (double)xlo[N3 + i] : 0.0);
-    out[i] = 0.5 * (p * p + mb.m2 * f * f + 0.25 * inv * (dx * dx + dy * dy + dz * dz));
-  }
+  EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * mb.N3 : x, nullptr, rho + (long long)blockIdx.z * mb.N3, nullptr, nullptr,
+                  N, a_chunk, mb.m2, mb.inv_scale / a2, 0.0, nullptr};
+  const int a0 = blockIdx.y * a_chunk;
+  energy_march<S, ED_QUAD, false>(A, task, a0, min(a0 + a_chunk, N));
 }
 
 // batched binning (blockIdx.y = batch entry), same fixed-point scheme as cf_spectrum.cu
@@ -910,12 +904,12 @@ static int spectra(cf_ensemble *E, double t, double *d_out, cudaStream_t st) {
   }
   for (auto &c : E->classes) {
     const int n = (int)c.members.size();
-    const long long N3 = (long long)c.N * c.N * c.N;
-    dim3 grid((unsigned)std::min<long long>((N3 + 255) / 256, 148LL * 4), n);
+    const int ch = energy_chunk(c.N, n);
+    const dim3 grid((unsigned)((energy_tasks(c.N) + 7) / 8), (unsigned)((c.N + ch - 1) / ch), n);
     if (E->word == 4)
-      k_ens_energy<float><<<grid, 256, 0, st>>>(E->dm, c.d_members, c.rho, c.N, a2);
+      k_ens_energy<float><<<grid, 256, 0, st>>>(E->dm, c.d_members, c.rho, c.N, ch, a2);
     else
-      k_ens_energy<double><<<grid, 256, 0, st>>>(E->dm, c.d_members, c.rho, c.N, a2);
+      k_ens_energy<double><<<grid, 256, 0, st>>>(E->dm, c.d_members, c.rho, c.N, ch, a2);
     CF_TRY_CUDA(cudaGetLastError());
     E->launches++;
     CF_TRY_CUFFT(cufftSetStream(c.plan, st));

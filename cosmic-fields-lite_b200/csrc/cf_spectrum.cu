@@ -5,8 +5,9 @@
 // :25).  Here every mode value is converted to a 128-bit fixed-point integer
 // whose scale is a power of two chosen from an order-independent upper bound on
 // any bin -- the largest mode value times the entry count (a max pass over the
-// modes), or for the density spectrum N^5 times the largest row sum of rho^2,
-// formed by the energy pass itself (Parseval) -- and the bins accumulate those
+// modes), or by Parseval a sum over the lattice that an earlier pass forms: of rho^2
+// in the energy pass for the density spectrum, of the state in the widening of an FP32_COMP
+// state for the mode spectrum -- and the bins accumulate those
 // integers with 64-bit integer atomics (carry propagated to the high word).
 // Integer addition is associative, so the bins are bit-reproducible, and the
 // sums are exact up to the fixed-point resolution (2^-126 of the bound).
@@ -17,78 +18,17 @@
 
 #include <cmath>
 
+#include "cf_energy.cuh"
 #include "cf_internal.cuh"
 
 namespace cfb {
 
-// ---- energy density -----------------------------------------------------
-// Potential term of the energy density by equation (ED_*):
-//   ED_QUAD    1/2 m^2 phi^2                                (src/equations_cuda.cu:332-369, lambda = 0)
-//   ED_LAMBDA  1/2 m^2 phi^2 + 1/4 lambda phi^4              (:332-369)
-//   ED_SQRT    m^2 f_a^2 (sqrt(1 + phi^2/f_a^2) - 1)         (:431-449)
-//   ED_CURV    1/2 m^2 phi^2 with e^{-2Psi} kinetic and e^{2Psi} gradient weights (:451-473)
-// and rho = 1/2 pi^2 w_k + 1/8 inv w_g sum_axes (phi_{+1} - phi_{-1})^2 + V
-// (src/equations.cpp:38-69, :106-138, :265-322 for the CPU twins).  `psi` holds
-// e^{2 Psi} - 1.  The sqrt potential is formed as m^2 phi^2 / (sqrt(1 + phi^2/f_a^2) + 1),
-// the same value without the cancellation of sqrt(1 + u) - 1 at small u.
-enum EdKind : int { ED_QUAD = 0, ED_LAMBDA = 1, ED_SQRT = 2, ED_CURV = 3 };
-
-// With `rowmax` set, the block also forms its row's sum of rho^2 (fixed order: the
-// thread's c values in turn, then a shuffle tree, then the warps in turn) and folds it
-// into *rowmax with an integer max of the bit pattern; N^2 times the largest row sum
-// bounds sum_x rho^2, which Parseval turns into a bound on every spectrum bin.
-template <typename S, int ED>
-__global__ void __launch_bounds__(128) k_energy(const S *__restrict__ x, const S *__restrict__ xlo,
-                                                const S *__restrict__ psi, double *__restrict__ rho, int N, double m2,
-                                                double inv, double q, unsigned long long *__restrict__ rowmax) {
-  // one lattice row (a, b) per block, threads along c: the row's neighbour rows are
-  // found once, only c wraps per site
-  double ss = 0.0;
-  const long long N3 = (long long)N * N * N;
-  const long long NN = (long long)N * N;
-  const int a = (int)(blockIdx.x / (unsigned)N), b = (int)(blockIdx.x - (unsigned)a * (unsigned)N);
-  const long long row = NN * a + (long long)N * b;
-  const long long rap = NN * (a + 1 == N ? 0 : a + 1) + (long long)N * b;
-  const long long ram = NN * (a == 0 ? N - 1 : a - 1) + (long long)N * b;
-  const long long rbp = NN * a + (long long)N * (b + 1 == N ? 0 : b + 1);
-  const long long rbm = NN * a + (long long)N * (b == 0 ? N - 1 : b - 1);
-  auto phi = [&](long long i) -> double {
-    double v = (double)x[i];
-    if (xlo) v += (double)xlo[i];
-    return v;
-  };
-  for (int c = threadIdx.x; c < N; c += blockDim.x) {
-    const long long i = row + c;
-    const int cp = c + 1 == N ? 0 : c + 1, cm = c == 0 ? N - 1 : c - 1;
-    const double dx = phi(rap + c) - phi(ram + c), dy = phi(rbp + c) - phi(rbm + c), dz = phi(row + cp) - phi(row + cm);
-    const double grad = dx * dx + dy * dy + dz * dz;
-    const double f = phi(i);
-    double p = (double)x[N3 + i];
-    if (xlo) p += (double)xlo[N3 + i];
-    double r;
-    if constexpr (ED == ED_CURV) {
-      const double e2 = 1.0 + (double)psi[i];
-      r = 0.5 * (p * p / e2 + m2 * f * f + e2 * 0.25 * inv * grad);
-    } else if constexpr (ED == ED_LAMBDA) {
-      r = 0.5 * (p * p + m2 * f * f + 0.25 * inv * grad) + 0.25 * q * f * f * f * f;
-    } else if constexpr (ED == ED_SQRT) {  // q = 1 / f_a^2
-      r = 0.5 * (p * p + 0.25 * inv * grad) + m2 * f * f / (sqrt(1.0 + f * f * q) + 1.0);
-    } else {
-      r = 0.5 * (p * p + m2 * f * f + 0.25 * inv * grad);
-    }
-    rho[i] = r;
-    ss += r * r;
-  }
-  if (!rowmax) return;  // uniform over the block
-  __shared__ double part[4];
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const double t = ((part[0] + part[1]) + part[2]) + part[3];
-    // non-negative doubles order like their bit patterns
-    atomicMax(rowmax, (unsigned long long)__double_as_longlong(t));
-  }
+template <typename S, int ED, bool MEAN>
+__global__ void __launch_bounds__(256) k_energy(const EnergyArgs<S> A) {
+  const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (task >= (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE)) return;  // whole warps
+  const int a0 = blockIdx.y * A.a_chunk;
+  energy_march<S, ED, MEAN>(A, task, a0, min(a0 + A.a_chunk, A.N));
 }
 
 // d rho / dt of the FRW Klein-Gordon equation (src/equations_cuda.cu:372-424):
@@ -136,6 +76,34 @@ __global__ void k_export_f32(const float *__restrict__ s, double *__restrict__ o
   const long long stride = (long long)gridDim.x * blockDim.x;
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < n2; i += stride)
     out[i] = (double)s[i] + (double)s[n2 + i];
+}
+
+// The same for the mode spectrum, with the largest block's sum of phi^2 + pi^2 / m^2 (fixed order,
+// an integer max of the bit pattern) in *blockmax: times the number of blocks it bounds the sum
+// over the lattice, and by Parseval, N^3 times that, the sum of the weighted mode values
+// |phi_k|^2 + |pi_k|^2 / (m^2 + k^2 / a^2), so the binning needs no pass over the modes to find
+// their maximum.
+__global__ void __launch_bounds__(256) k_export_bound_f32(const float *__restrict__ s, double *__restrict__ out,
+                                                          long long n2, double inv_m2,
+                                                          unsigned long long *__restrict__ blockmax) {
+  const long long stride = 2LL * gridDim.x * blockDim.x;
+  double ss = 0.0;
+  for (long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < n2; i += stride) {
+    const float2 h = *reinterpret_cast<const float2 *>(s + i), l = *reinterpret_cast<const float2 *>(s + n2 + i);
+    const double2 v = make_double2((double)h.x + (double)l.x, (double)h.y + (double)l.y);
+    *reinterpret_cast<double2 *>(out + i) = v;
+    const double q = v.x * v.x + v.y * v.y;
+    ss += 2 * i < n2 ? q : q * inv_m2;
+  }
+  __shared__ double part[8];
+  for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
+  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = part[0];
+    for (int w = 1; w < 8; ++w) t += part[w];
+    atomicMax(blockmax, (unsigned long long)__double_as_longlong(t));
+  }
 }
 
 // FP64 [phi | pi] -> FP32_COMP state.
@@ -501,53 +469,69 @@ int power_spectrum_s2(cf_ctx *ctx, const double *d_f, double *d_out, cudaStream_
   return bin_spectrum(ctx, false, 1.0, d_out, st);
 }
 
-static const double *state_as_f64(cf_ctx *ctx, const void *d_state, cudaStream_t st, int *err) {
-  *err = CF_OK;
-  if (ctx->p.precision == CF_FP64) return (const double *)d_state;
-  const long long n2 = 2 * ctx->N3;
-  k_export_f32<<<grid_for(n2), 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2);
-  if (cudaGetLastError() != cudaSuccess) {
-    set_error("state export launch failed");
-    *err = CF_ERR_CUDA;
-  }
-  ctx->launches++;
-  return ctx->spec_field;
-}
-
 int mode_power_spectrum_s2(cf_ctx *ctx, const void *d_state, double a_t, double *d_out, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 2));
-  int err;
-  const double *x = state_as_f64(ctx, d_state, st, &err);
-  CF_TRY(err);
+  const double *x = (const double *)d_state;
+  long long bound = 0;
+  if (ctx->p.precision != CF_FP64) {
+    // The state is widened for the transform anyway, so its sums come along and bound the bins
+    // (N = 512: the 0.49 ms of the max pass) unless the bound could be more than 2^20 above the
+    // sum of the mode values (k_max^2 against a^2 m^2): the fixed point keeps 2^-106 of that
+    // sum, more than the FP64 results resolve.  An FP64 state would need a pass of its own.
+    const long long n2 = 2 * ctx->N3;
+    const double m2 = ctx->p.m * ctx->p.m, k = 3.14159265358979323846 * ctx->N / ctx->p.L;
+    const unsigned blocks = grid_for(n2 / 2);
+    if (3.0 * k * k < 1048576.0 * m2 * a_t * a_t) {
+      bound = ctx->N3 * (long long)blocks;
+      CF_TRY_CUDA(cudaMemsetAsync(ctx->maxbits, 0, sizeof(unsigned long long), st));
+      k_export_bound_f32<<<blocks, 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2, 1.0 / m2, ctx->maxbits);
+    } else {
+      k_export_f32<<<grid_for(n2), 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2);
+    }
+    CF_LAUNCHED(ctx);
+    x = ctx->spec_field;
+  }
   CF_TRY_CUFFT(cufftSetStream(ctx->plan_d2z2, st));
   {
     ProfScope ps(ctx, CF_PROF_SPECTRUM, st);
     CF_TRY_CUFFT(cufftExecD2Z(ctx->plan_d2z2, (cufftDoubleReal *)x, (cufftDoubleComplex *)ctx->spec_hc));
   }
-  return bin_spectrum(ctx, true, a_t, d_out, st);
+  return bin_spectrum(ctx, true, a_t, d_out, st, bound);
 }
 
+// What the energy passes write: rho (with rowmax optional), or its mean and slice.
+struct EnergyOut {
+  double *rho = nullptr;
+  unsigned long long *rowmax = nullptr;
+  double *slice = nullptr, *mean = nullptr;
+};
+
 template <typename S, int ED>
-static void launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, double *d_rho, double m2, double inv,
-                          double q, unsigned long long *rowmax, cudaStream_t st) {
+static void launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
+                          double q, cudaStream_t st) {
   const long long N3 = ctx->N3;
+  const int N = (int)ctx->N;
   const S *x = (const S *)d_state;
-  k_energy<S, ED><<<(unsigned)(ctx->N * ctx->N), 128, 0, st>>>(x, sizeof(S) == 4 ? x + 2 * N3 : nullptr,
-                                                               (const S *)psi, d_rho, (int)ctx->N, m2, inv, q, rowmax);
+  EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * N3 : x, (const S *)psi, o.rho, o.slice, o.mean, N, N, m2, inv, q, o.rowmax};
+  const unsigned gx = (unsigned)((energy_tasks(N) + 7) / 8);
+  if (!o.rho) {
+    k_energy<S, ED, true><<<gx, 256, 0, st>>>(A);
+  } else {
+    A.a_chunk = energy_chunk(N, 1);
+    k_energy<S, ED, false><<<dim3(gx, (unsigned)((N + A.a_chunk - 1) / A.a_chunk)), 256, 0, st>>>(A);
+  }
 }
 
 template <int ED>
-static void launch_energy_p(cf_ctx *ctx, const void *d_state, const void *psi, double *d_rho, double m2, double inv,
-                            double q, unsigned long long *rowmax, cudaStream_t st) {
+static void launch_energy_p(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
+                            double q, cudaStream_t st) {
   if (ctx->p.precision == CF_FP32_COMP)
-    launch_energy<float, ED>(ctx, d_state, psi, d_rho, m2, inv, q, rowmax, st);
+    launch_energy<float, ED>(ctx, d_state, psi, o, m2, inv, q, st);
   else
-    launch_energy<double, ED>(ctx, d_state, psi, d_rho, m2, inv, q, rowmax, st);
+    launch_energy<double, ED>(ctx, d_state, psi, o, m2, inv, q, st);
 }
 
-// `rowmax` (optional, zeroed by the caller): receives the largest row sum of rho^2.
-static int energy_density_b(cf_ctx *ctx, const void *d_state, double t, double *d_rho, unsigned long long *rowmax,
-                            cudaStream_t st) {
+static int energy_density_b(cf_ctx *ctx, const void *d_state, double t, const EnergyOut &o, cudaStream_t st) {
   double inv, H;
   stage_coeffs(ctx->p, t, &inv, &H);
   const double m2 = ctx->p.m * ctx->p.m;
@@ -559,19 +543,21 @@ static int energy_density_b(cf_ctx *ctx, const void *d_state, double t, double *
   if (eq == CF_EQ_FIXED_CURVATURE_FRW) ps = ctx->fixed_e2m1;
   ProfScope prof(ctx, CF_PROF_SPECTRUM, st);
   if (ps)
-    launch_energy_p<ED_CURV>(ctx, d_state, ps, d_rho, m2, inv, 0.0, rowmax, st);
+    launch_energy_p<ED_CURV>(ctx, d_state, ps, o, m2, inv, 0.0, st);
   else if (eq == CF_EQ_LAMBDA_FRW)
-    launch_energy_p<ED_LAMBDA>(ctx, d_state, nullptr, d_rho, m2, inv, ctx->p.lambda, rowmax, st);
+    launch_energy_p<ED_LAMBDA>(ctx, d_state, nullptr, o, m2, inv, ctx->p.lambda, st);
   else if (eq == CF_EQ_SQRT_FRW)
-    launch_energy_p<ED_SQRT>(ctx, d_state, nullptr, d_rho, m2, inv, 1.0 / (ctx->p.f_a * ctx->p.f_a), rowmax, st);
+    launch_energy_p<ED_SQRT>(ctx, d_state, nullptr, o, m2, inv, 1.0 / (ctx->p.f_a * ctx->p.f_a), st);
   else
-    launch_energy_p<ED_QUAD>(ctx, d_state, nullptr, d_rho, m2, inv, 0.0, rowmax, st);
+    launch_energy_p<ED_QUAD>(ctx, d_state, nullptr, o, m2, inv, 0.0, st);
   CF_LAUNCHED(ctx);
   return CF_OK;
 }
 
 int energy_density(cf_ctx *ctx, const void *d_state, double t, double *d_rho, cudaStream_t st) {
-  return energy_density_b(ctx, d_state, t, d_rho, nullptr, st);
+  EnergyOut o;
+  o.rho = d_rho;
+  return energy_density_b(ctx, d_state, t, o, st);
 }
 
 int dot_energy_density(cf_ctx *ctx, const void *d_state, double t, double *d_out, cudaStream_t st) {
@@ -602,9 +588,19 @@ __global__ void k_axis_mean(const double *__restrict__ f, double *__restrict__ o
 }
 
 int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, double *d_avg, cudaStream_t st) {
+  const long long NN = ctx->N * ctx->N;
+  // With a warp per SM sub-partition or more from one chunk of all planes, the energy pass
+  // sums over a itself and the density is not written; smaller lattices need the chunks
+  // (N = 512: 0.96 ms against 1.30 for the density and a pass over it).
+  if (energy_tasks((int)ctx->N) >= 148LL * 8) {
+    EnergyOut o;
+    o.slice = d_slice;
+    o.mean = d_avg;
+    if (!d_slice && !d_avg) return CF_OK;
+    return energy_density_b(ctx, d_state, t, o, st);
+  }
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
   CF_TRY(energy_density(ctx, d_state, t, ctx->spec_field, st));
-  const long long NN = ctx->N * ctx->N;
   if (d_slice)
     CF_TRY_CUDA(cudaMemcpyAsync(d_slice, ctx->spec_field, NN * sizeof(double), cudaMemcpyDeviceToDevice, st));
   if (d_avg) {
@@ -616,19 +612,22 @@ int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, 
 }
 
 // The fixed-point scale comes from the energy pass: by Parseval the weighted HC
-// values of rho sum to N^3 sum_x rho^2 <= N^5 max_row sum_c rho^2, so no bin can
-// exceed that bound, and the binning needs no pass of its own to find a maximum.
+// values of rho sum to N^3 sum_x rho^2 <= N^5 ceil(N/64) times the largest sum over 64
+// sites of a row, so no bin can exceed that bound, and the binning needs no pass of its own to find a maximum.
 int density_spectrum_s2(cf_ctx *ctx, const void *d_state, double t, double *d_out, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
   CF_TRY_CUDA(cudaMemsetAsync(ctx->maxbits, 0, sizeof(unsigned long long), st));
-  CF_TRY(energy_density_b(ctx, d_state, t, ctx->spec_field, ctx->maxbits, st));
+  EnergyOut o;
+  o.rho = ctx->spec_field;
+  o.rowmax = ctx->maxbits;
+  CF_TRY(energy_density_b(ctx, d_state, t, o, st));
   CF_TRY_CUFFT(cufftSetStream(ctx->plan_d2z1, st));
   {
     ProfScope ps(ctx, CF_PROF_SPECTRUM, st);
     CF_TRY_CUFFT(cufftExecD2Z(ctx->plan_d2z1, (cufftDoubleReal *)ctx->spec_field, (cufftDoubleComplex *)ctx->spec_hc));
   }
   const long long N = ctx->N;
-  return bin_spectrum(ctx, false, 1.0, d_out, st, N * N * N * N * N);
+  return bin_spectrum(ctx, false, 1.0, d_out, st, N * N * N * N * N * ((N + ED_TILE - 1) / ED_TILE));
 }
 
 int s2_to_shells(cf_ctx *ctx, double *d_shells, int64_t *d_counts, cudaStream_t st) {

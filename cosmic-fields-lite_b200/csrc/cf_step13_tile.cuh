@@ -166,8 +166,8 @@ __device__ __forceinline__ void step13_tile(const StepArgs<S> &A, int c0, int b0
   };
   // the curvature of two stages at the sites of a row
   auto couple = [&](auto &ca, auto &cb, int ka, int kb, long long site, int ai, const auto &cc) {
-    constexpr int VV = sizeof(ca.ps.v) / sizeof(S);
     if constexpr (EqOf<EQ>::coupled) {
+      constexpr int VV = sizeof(ca.ps.v) / sizeof(S);
       const int row = EqOf<EQ>::coarse ? __ldg(A.cmap + ai) : 0;
       load_coupling<EQ, S, VV>(ca, A.psi[ka], A.dpsi[ka], site, A.M, row, cc);
       if constexpr (EQ == EQ_FIXED)
