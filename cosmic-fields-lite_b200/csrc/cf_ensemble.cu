@@ -569,6 +569,38 @@ static int build_step_items(cf_ensemble *E) {
   return E->sshape ? step_items_t<double, 1>(E) : step_items_t<double, 0>(E);
 }
 
+// The step shape and a-chunk an ensemble starts with (cf_ensemble_autotune times them
+// instead): the least time by the model of step_a_chunk (cf_step.cu) over the whole work list.
+// An item takes its planes, 4 halo planes and about 1.5 planes of start-up; a list longer than
+// the resident CTAs takes its sum over them and, for the uneven end, 3/4 of the longest
+// item; one that fits takes its longest item, by measurement 1.2 times as long as in a list of
+// several waves (the CTAs of an SM stay in step).  Against 128 x 8 tiles of 32 planes for all (ms per 25 steps, FP32, density spectra
+// included): 4 x (64, 96, 128) 5.05 -> 4.35, 3 x (40, 64, 72) 2.37 -> 1.41, 96 + 96 + 128 2.05 -> 1.65.
+template <typename S, int SS>
+static double step_list_cost(const cf_ensemble *E, int chunk) {
+  using SH = EnsStepShape<S, SS>;
+  constexpr int TW = SH::TX * VecT<S>::n;
+  double n = 0.0, sum = 0.0, longest = 0.0;
+  for (const EnsMember &m : E->hm) {
+    const double tiles = (double)((m.N + TW - 1) / TW) * ((m.N + SH::TY - 1) / SH::TY);
+    n += tiles * ((m.N + chunk - 1) / chunk);
+    sum += tiles * (m.N + 5.5 * ((m.N + chunk - 1) / chunk));
+    longest = std::max(longest, std::min(chunk, m.N) + 5.5);
+  }
+  const double slots = 148.0 * SH::MB;
+  if (n <= slots) return 1.2 * longest * std::max(0.62, 0.27 + std::ceil(n / 148.0) / SH::MB);
+  return sum / slots * 1.27 + 0.75 * longest;
+}
+template <typename S>
+static void pick_step_list(cf_ensemble *E) {
+  double best = -1.0;
+  for (int chunk : {8, 12, 16, 24, 32, 48, 64}) {
+    const double c[2] = {step_list_cost<S, 0>(E, chunk), step_list_cost<S, 1>(E, chunk)};
+    for (int k = 0; k < 2; ++k)
+      if (best < 0.0 || c[k] < best) best = c[k], E->sshape = k, E->schunk = chunk;
+  }
+}
+
 static int ensure_coef(cf_ensemble *E, double t0, double dt, long long nsteps_total, cudaStream_t st) {
   if (E->d_coef && E->coef_cap >= nsteps_total && E->coef_t0 == t0 && E->coef_dt == dt) return CF_OK;
   std::vector<EnsCoef> h((size_t)(4 * nsteps_total));
@@ -997,6 +1029,12 @@ int cf_ensemble_create(const cf_params *members, int count, cf_ensemble **out) {
   cudaMemset(E->d_step, 0, sizeof(long long));
   build_items(E);
   int s = upload_items(E);
+  if (E->stencil == 7) {
+    if (E->word == 4)
+      pick_step_list<float>(E);
+    else
+      pick_step_list<double>(E);
+  }
   if (s == CF_OK) s = build_step_items(E);
   if (s != CF_OK) {
     cf_ensemble_destroy(E);
