@@ -340,7 +340,7 @@ int launch_forward_stage(cf_ctx *ctx, int stage, const void *yin, void *yout, vo
                          double cy, double dt6, cudaStream_t st);
 // One step from one state into another (cf_step.cu), as rk4_steps takes it in place.
 int rk4_step_to(cf_ctx *ctx, const void *from, void *to, double t0, double dt, int64_t step, cudaStream_t st);
-int step_a_chunk(int N, int tiles_xy, int per_sm, int halo);
+int step_a_chunk(int N, int tiles_xy, int per_sm, int halo, double latency);
 
 }  // namespace cfb
 
@@ -389,7 +389,7 @@ static int launch_adj_h(cf_adjoint *adj, const AdjArgs<S> &A, cudaStream_t st) {
 // Tiles and planes per CTA of the whole reverse step.
 static dim3 adj_step_grid(long long N, int *a_chunk) {
   const unsigned gx = ceil_div(N, AS_TX * 2), gy = ceil_div(N, AS_TY);
-  *a_chunk = step_a_chunk((int)N, (int)(gx * gy), AS_MB, 4);
+  *a_chunk = step_a_chunk((int)N, (int)(gx * gy), AS_MB, 4, step_latency(8, false));
   return dim3(gx, gy, ceil_div(N, *a_chunk));
 }
 

@@ -588,7 +588,7 @@ static double step_list_cost(const cf_ensemble *E, int chunk) {
     longest = std::max(longest, std::min(chunk, m.N) + 5.5);
   }
   const double slots = 148.0 * SH::MB;
-  if (n <= slots) return 1.2 * longest * std::max(0.62, 0.27 + std::ceil(n / 148.0) / SH::MB);
+  if (n <= slots) return 1.2 * longest * std::max(step_latency(sizeof(S), false), 0.27 + std::ceil(n / 148.0) / SH::MB);
   return sum / slots * 1.27 + 0.75 * longest;
 }
 template <typename S>

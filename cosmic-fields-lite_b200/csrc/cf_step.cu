@@ -420,18 +420,18 @@ __global__ void __launch_bounds__(StepShape<S, EQ>::TX *step_threads_y<S, EQ>(),
 // chunks of at most 72 planes, as many as minimise the time of the waves they make.  A
 // CTA marches over its chunk and `halo` more planes (each chunk forms them again) and
 // starts up in about 1.5 planes' time; with c CTAs on the fullest SM a plane takes 0.27 + c /
-// per_sm of the time it takes per CTA on a full one, and never less than 0.62 (latency; from
-// sweeps of the chunk at N = 48 ... 256, FP64: 0.76 us with one CTA per SM, 1.66 us with
-// four).  Against halving from 64 until the grid is six CTAs per SM deep: N = 128 FP64 39.9
-// -> 33.3 us per step, FP32 13-point 79.8 -> 68.7 us, N = 48 and N = 256 the same chunks.
-int step_a_chunk(int N, int tiles_xy, int per_sm, int halo) {
+// per_sm of the time it takes per CTA on a full one, and never less than `latency` (below).
+// Against halving from 64 until the grid is six CTAs per SM deep: N = 128 FP64 39.9
+// -> 31.3 us per step, comoving FP32 43.9 -> 34.6 us, FP32 13-point 79.8 -> 39.6 us (with its new
+// pass), N = 32 FP64 6.8 -> 5.3 us, N = 48 and N = 256 the same chunks.
+int step_a_chunk(int N, int tiles_xy, int per_sm, int halo, double latency) {
   const double slots = 148.0 * per_sm;
   int best = 1;
   double best_cost = 0.0;
-  for (int nc = (N + 71) / 72; nc <= (N + 1) / 2; ++nc) {
+  for (int nc = (N + 71) / 72; nc <= N; ++nc) {
     const int chunk = (N + nc - 1) / nc, chunks = (N + chunk - 1) / chunk;
     const double n = (double)tiles_xy * chunks, w = std::floor(n / slots), c = std::ceil((n - w * slots) / 148.0);
-    const double last = c > 0 ? std::max(0.62, 0.27 + c / per_sm) : 0.0;  // the wave that is not full
+    const double last = c > 0 ? std::max(latency, 0.27 + c / per_sm) : 0.0;  // the wave that is not full
     const double cost = (chunk + halo + 1.5) * (w * 1.27 + last);
     if (best_cost == 0.0 || cost < best_cost) best_cost = cost, best = chunk;
   }
@@ -459,7 +459,7 @@ static int launch_step_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
   constexpr int TYs = StepShape<S, EQ>::TY;
   StepArgs<S> A = A0;
   unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, TYs);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4);
+  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4, step_latency(sizeof(S), EqOf<EQ>::coupled));
   step_coefs_f32(A);
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
@@ -528,7 +528,7 @@ static int launch_step13_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) 
   using SM = Step13Smem<S, SH::TX, SH::TY>;
   StepArgs<S> A = A0;
   const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, SH::TY);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8);
+  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8, step_latency(sizeof(S), EqOf<EQ>::coupled));
   for (double &inv : A.inv) inv = lap_coef<2>(inv);  // the 13-point sum's 1/12
   step_coefs_f32(A);
   const dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));

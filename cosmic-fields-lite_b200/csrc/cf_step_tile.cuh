@@ -290,6 +290,11 @@ constexpr int step_ring_rows(int TXv, int TYv) {
   return r;
 }
 
+// The least time of a plane, in the units of step_a_chunk (1.27 on a full SM): a lone CTA's chain of
+// dependent steps.  Measured per plane with one CTA per SM against a full one: FP64 0.76 / 1.66
+// us (5 of 20 warps), FP32 1.19 / 1.59 us, comoving 2.16 / 2.56 us (10 of 20 warps).
+constexpr double step_latency(size_t word, bool coupled) { return word == 8 ? 0.62 : (coupled ? 1.05 : 0.95); }
+
 __device__ __forceinline__ void step_barrier(int threads) { asm volatile("bar.sync 1, %0;\n" ::"r"(threads) : "memory"); }
 
 template <typename S, int EQ, int TXv, int TYv, bool FULL = false>
