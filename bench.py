@@ -45,10 +45,10 @@ WORKLOAD = dict(workload="comoving-curvature KG, radiation FRW, N=512^3, L=512, 
 # Algorithmic HBM bytes per site and RK4 step, by route.
 def stage_bytes_per_site(precision, comoving, route="step"):
     """Algorithmic HBM bytes per site-update of one RK4 step.
-    route "step" (one whole-step pass, the 7-point default): the state in and out --
+    route "step" (one whole-step pass, the default for both stencils): the state in and out --
     FP64 phi, pi (4 words), FP32-comp hi and lo of phi, pi (8 words) -- plus Psi, dPsi
-    at three stage times (+6 words, comoving).  route "pair" (stages 1+2, 3+4; the
-    13-point route): FP64 6 + 8 words, FP32-comp 6 + 12, Psi at four stage times +8.
+    at three stage times (+6 words, comoving).  route "pair" (stages 1+2, 3+4): FP64
+    6 + 8 words, FP32-comp 6 + 12, Psi at four stage times +8.
     route "stage" (four single-stage passes): FP64 32, FP32-comp 38, +8."""
     w = 8 if precision == "fp64" else 4
     if route == "step":
@@ -659,7 +659,7 @@ def run_product(args):
         c2, s2_ = make_case(N, L, prec, stencil, com)
         t2, _, p2 = time_steps(c2, s2_, ks, args.warmup, profile=True)
         sm = sum(p2[k][1] for k in cfb200.STEP_KINDS)
-        bb = stage_bytes_per_site(prec, com, "step" if stencil == 7 else "pair")
+        bb = stage_bytes_per_site(prec, com, "step")
         secondary[name] = {"value": world * N ** 3 * ks / (max_over_ranks(t2, pg) * 1e-3),
                            "ms_per_step": t2 / ks,
                            "stage_kernels_gbs": bb * N ** 3 * ks / (sm * 1e-3) / 1e9}
