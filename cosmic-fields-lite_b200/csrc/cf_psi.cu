@@ -1259,7 +1259,7 @@ __global__ void k_copy_convert(const double *__restrict__ in, S *__restrict__ ou
 // a with the transfer factors applied as R is read (once, for both fields), along b in place,
 // along c with e^{2 Psi} - 1 applied as Psi is written: 9 half-complex arrays of traffic
 // against 15 for the transfer kernel, a cuFFT Z2D and the exponential.  Per refresh, ms: N = 256
-// 0.455 -> 0.38, N = 384 2.32 -> 1.35, N = 512 3.87 -> 3.27 (two fields).
+// 0.454 -> 0.367, N = 384 2.32 -> 1.31, N = 512 3.87 -> 3.21 (two fields).
 template <int N>
 struct PsiTileA {  // lines along a at one b, L values of k from k0; both fields of it
   const C64 *R;

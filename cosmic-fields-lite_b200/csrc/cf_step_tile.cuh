@@ -54,10 +54,10 @@
 // register budget without spills), and both meet at one named barrier per plane.
 //
 // What bounds it: latency and shared-memory bandwidth, not HBM -- at N = 256 the FP32 FRW
-// pass issues in 54% of the cycles and the shared-memory pipe is busy in 71% (FP64: 89%).
+// pass issues in 51% of the cycles and the shared-memory pipe is busy in 69% (FP64: 82%).
 // Measured against the form that read every stencil point from shared memory and formed
 // ya_phi per point (N = 512, ms per step, FP32: FRW 1.18 -> 1.06, fixed Psi 1.40 -> 1.21,
-// comoving with its Psi refreshes 2.55 -> 2.35; FP64 at N = 256: FRW 0.233 -> 0.192, sqrt
+// comoving with its Psi refreshes 2.34 -> 2.09; FP64 at N = 256: FRW 0.233 -> 0.192, sqrt
 // potential 0.276 -> 0.266).  Measured and not taken: 2 floats or 1 double per thread
 // (twice the warps: 10 to 20% slower), c-neighbours by warp shuffles (spills), 128 x 16 tiles
 // at 1 CTA per SM.
