@@ -220,8 +220,6 @@ int psi_pipe_fill(cf_ctx *ctx, double t, const double *keep, int nkeep);
 int psi_pipe_use(cf_ctx *ctx, double t, cudaStream_t stream, const void **psi, const void **dpsi);
 int psi_pipe_step_done(cf_ctx *ctx, cudaStream_t stream);
 int psi_pipe_end(cf_ctx *ctx, cudaStream_t stream);
-// The twiddle tables of cf_fft3.cuh (ctx->fft_tw).
-int ensure_fft_tw(cf_ctx *ctx);
 // Psi and dPsi at t, widened to FP64, into d_out (2 N^3 doubles).
 int psi_fields(cf_ctx *ctx, double t, double *d_out, cudaStream_t stream);
 // CF_PSI_* route the next Psi refresh takes.

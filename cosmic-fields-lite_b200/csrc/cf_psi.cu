@@ -1347,20 +1347,27 @@ __global__ void __launch_bounds__(RowShape<N / 2>::T) k_psi_along_c(const C64 *_
   });
 }
 
-int ensure_fft_tw(cf_ctx *ctx) {
+// Kept only once the copy has landed: later refreshes may run on another stream.
+static int ensure_fft_tw(cf_ctx *ctx, cudaStream_t st) {
   if (ctx->fft_tw) return CF_OK;
   const int N = (int)ctx->N, M = N / 2;
   std::vector<double2> t((size_t)N + M);
   const long double two_pi = 6.28318530717958647692528676655900577L;
   for (int j = 0; j < N; ++j) t[j] = make_double2((double)cosl(two_pi * j / N), (double)sinl(two_pi * j / N));
   for (int j = 0; j < M; ++j) t[N + j] = t[2 * j];
-  if (cudaMalloc((void **)&ctx->fft_tw, t.size() * sizeof(double2)) != cudaSuccess) {
+  double2 *tw = nullptr;
+  if (cudaMalloc((void **)&tw, t.size() * sizeof(double2)) != cudaSuccess) {
     cudaGetLastError();
-    ctx->fft_tw = nullptr;
     set_error("cudaMalloc twiddle table failed");
     return CF_ERR_NOMEM;
   }
-  CF_TRY_CUDA(cudaMemcpy(ctx->fft_tw, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice));
+  cudaError_t e = cudaMemcpyAsync(tw, t.data(), t.size() * sizeof(double2), cudaMemcpyHostToDevice, st);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+  if (e != cudaSuccess) {
+    cudaFree(tw);
+    CF_TRY_CUDA(e);
+  }
+  ctx->fft_tw = tw;
   return CF_OK;
 }
 
@@ -1387,7 +1394,7 @@ static int full_synthesis_n(cf_ctx *ctx, double *out, cudaStream_t st) {
 }
 
 static int full_synthesis(cf_ctx *ctx, void *out, cudaStream_t st) {
-  CF_TRY(ensure_fft_tw(ctx));
+  CF_TRY(ensure_fft_tw(ctx, st));
   switch (ctx->N) {
     case 64: return full_synthesis_n<64>(ctx, (double *)out, st);
     case 96: return full_synthesis_n<96>(ctx, (double *)out, st);
