@@ -459,7 +459,11 @@ static int launch_step_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
   constexpr int TYs = StepShape<S, EQ>::TY;
   StepArgs<S> A = A0;
   unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, TYs);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4, step_latency(sizeof(S), EqOf<EQ>::coupled));
+  // The least time is one CTA's, whatever the CTAs per SM: the FP64 sqrt potential at 3 instead
+  // of 4 has it at 4/3 of a full SM's share (N = 64 12.1 -> 10.3 us, N = 48 8.8 -> 8.0).
+  const double few = (sizeof(S) == 8 && EQ == EQ_SQRT) ? 4.0 / StepShape<S, EQ>::MB : 1.0;
+  A.a_chunk =
+      step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4, few * step_latency(sizeof(S), EqOf<EQ>::coupled));
   step_coefs_f32(A);
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
@@ -761,9 +765,20 @@ int rk4_step_buffers(cf_ctx *ctx, void *d_state, void *acc, void *ya, void *yb, 
   return rk4_step_buffers_t<double>(ctx, d_state, acc, ya, yb, t, dt, st);
 }
 
-// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).
+// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).  From N =
+// 72 to 120 the FP32 13-point comoving pass, whose CTAs take an SM each, leaves the Psi
+// refreshes beside it no room, and a march of its few planes costs as much as two of the
+// paired passes': 10 steps in one call, us per step paired / whole, N = 80 96 / 106, 96 108 /
+// 111, 112 151 / 161, 120 174 / 183, but 128 95 / 86 and 144 263 / 240; at 48 and 64 launches
+// bound both (75 / 75, 52 / 52) and one step per call is faster whole (91 / 86, 78 / 74).  Fixed Psi, which
+// refreshes nothing, loses only at 88 and 96, where the paired passes' grids are still one
+// wave and the whole pass has two 64-wide tiles per row: 80 25.2 / 23.6, 88 25.5 / 27.8, 96 26.6 /
+// 27.6, 104 40.9 / 33.9.
 static bool whole_step_route(const cf_ctx *ctx) {
-  return !(ctx->p.flags & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS));
+  if (ctx->p.flags & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS)) return false;
+  if (ctx->p.stencil != 13 || ctx->p.precision != CF_FP32_COMP) return true;
+  const int eq = shape_of(ctx->p.equation);
+  return !((eq == EQ_COMOV && ctx->N > 64 && ctx->N < 128) || (eq == EQ_FIXED && ctx->N > 80 && ctx->N <= 96));
 }
 
 int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, int64_t nsteps, cudaStream_t st) {
