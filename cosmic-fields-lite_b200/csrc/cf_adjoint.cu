@@ -357,6 +357,8 @@ struct cf_adjoint {
   double *dm_partial = nullptr;
   long long dm_slots = 0;
   double dm_direct = 0.0;
+  dim3 grid;        // of the whole reverse step (7-point), and its planes per CTA
+  int a_chunk = 0;
 };
 
 namespace cfb {
@@ -393,13 +395,9 @@ static dim3 adj_step_grid(long long N, int *a_chunk) {
   return dim3(gx, gy, ceil_div(N, *a_chunk));
 }
 
-static long long adj_cta_count(const cf_ctx *ctx) {
-  const long long N = ctx->N;
-  if (ctx->p.stencil == 7) {
-    int chunk;
-    const dim3 g = adj_step_grid(N, &chunk);
-    return (long long)g.x * g.y * g.z;
-  }
+static long long adj_cta_count(const cf_adjoint *a) {
+  const long long N = a->ctx->N;
+  if (a->ctx->p.stencil == 7) return (long long)a->grid.x * a->grid.y * a->grid.z;
   return (long long)ceil_div(N, ATX * 2) * (N / ATY) * ceil_div(N, 16);
 }
 
@@ -418,10 +416,9 @@ static int launch_adj_step_t(cf_ctx *ctx, const AdjStepArgs<S> &A, dim3 grid, cu
 }
 
 template <typename S>
-static int launch_adj_step(cf_ctx *ctx, AdjStepArgs<S> A, cudaStream_t st) {
-  const dim3 grid = adj_step_grid(A.N, &A.a_chunk);
-  if (A.N % (AS_TX * 2) == 0 && A.N % AS_TY == 0) return launch_adj_step_t<S, true>(ctx, A, grid, st);
-  return launch_adj_step_t<S, false>(ctx, A, grid, st);
+static int launch_adj_step(const cf_adjoint *a, const AdjStepArgs<S> &A, cudaStream_t st) {
+  if (A.N % (AS_TX * 2) == 0 && A.N % AS_TY == 0) return launch_adj_step_t<S, true>(a->ctx, A, a->grid, st);
+  return launch_adj_step_t<S, false>(a->ctx, A, a->grid, st);
 }
 
 int adjoint_create(cf_ctx *ctx, int64_t nsteps, int64_t every, cf_adjoint **out) {
@@ -448,7 +445,8 @@ int adjoint_create(cf_ctx *ctx, int64_t nsteps, int64_t every, cf_adjoint **out)
   ok = ok && alloc((void **)&a->lam, 2 * fb) && alloc((void **)&a->ka, 2 * fb) && alloc((void **)&a->rb, fb);
   if (ctx->p.stencil != 7)  // the single-stage route
     ok = ok && alloc(&a->Y, 3 * sb) && alloc((void **)&a->kb, 2 * fb) && alloc((void **)&a->accb, 2 * fb);
-  a->dm_slots = std::max<long long>(adj_cta_count(ctx), 148 * 16);
+  if (ctx->p.stencil == 7) a->grid = adj_step_grid(ctx->N, &a->a_chunk);
+  a->dm_slots = std::max<long long>(adj_cta_count(a), 148 * 16);
   ok = ok && alloc((void **)&a->dm_partial, sizeof(double) * (size_t)a->dm_slots);
   if (!ok) {
     cudaGetLastError();
@@ -555,6 +553,7 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
   const bool whole = ctx->p.stencil == 7;
   AdjStepArgs<S> W{};
   W.N = (int)ctx->N;
+  W.a_chunk = a->a_chunk;
   W.N3 = N3;
   W.m2 = ctx->p.m * ctx->p.m;
   W.two_m = 2.0 * ctx->p.m;
@@ -592,7 +591,7 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
         W.lam = a->lam;
         W.out = a->ka;
         W.x = x;
-        CF_TRY(launch_adj_step<S>(ctx, W, st));
+        CF_TRY(launch_adj_step<S>(a, W, st));
         std::swap(a->lam, a->ka);
         continue;
       }

@@ -90,6 +90,7 @@ struct cf_ctx {
 
   // RK4 temporaries (storage type): acc and ping-pong stage inputs, 2N^3 words each.
   void *acc = nullptr, *ya = nullptr, *yb = nullptr;
+  int step_chunk = 0;  // planes per CTA of this context's whole-step pass (step_a_chunk), once known
 
   // Comoving curvature: R_fft in the storage type's complex HC, the transfer
   // outputs (2 HC arrays) and the cached (Psi, dPsi) slots: three allocated with the

@@ -423,7 +423,8 @@ __global__ void __launch_bounds__(StepShape<S, EQ>::TX *step_threads_y<S, EQ>(),
 // per_sm of the time it takes per CTA on a full one, and never less than `latency` (below).
 // Against halving from 64 until the grid is six CTAs per SM deep: N = 128 FP64 39.9
 // -> 31.3 us per step, comoving FP32 43.9 -> 34.6 us, FP32 13-point 79.8 -> 39.6 us (with its new
-// pass), N = 32 FP64 6.8 -> 5.3 us, N = 48 and N = 256 the same chunks.
+// pass).  The search costs 0.7 us of host time at N = 48 and 6.8 at N = 512, so its answer is kept
+// (cf_ctx::step_chunk, cf_adjoint::grid): per step it was in the way of one-step calls.
 int step_a_chunk(int N, int tiles_xy, int per_sm, int halo, double latency) {
   const double slots = 148.0 * per_sm;
   int best = 1;
@@ -462,8 +463,10 @@ static int launch_step_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
   // The least time is one CTA's, whatever the CTAs per SM: the FP64 sqrt potential at 3 instead
   // of 4 has it at 4/3 of a full SM's share (N = 64 12.1 -> 10.3 us, N = 48 8.8 -> 8.0).
   const double few = (sizeof(S) == 8 && EQ == EQ_SQRT) ? 4.0 / StepShape<S, EQ>::MB : 1.0;
-  A.a_chunk =
-      step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4, few * step_latency(sizeof(S), EqOf<EQ>::coupled));
+  if (!ctx->step_chunk)
+    ctx->step_chunk =
+        step_a_chunk(A.N, (int)(gx * gy), StepShape<S, EQ>::MB, 4, few * step_latency(sizeof(S), EqOf<EQ>::coupled));
+  A.a_chunk = ctx->step_chunk;
   step_coefs_f32(A);
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, CF_PROF_STEP, st);
@@ -532,7 +535,9 @@ static int launch_step13_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) 
   using SM = Step13Smem<S, SH::TX, SH::TY>;
   StepArgs<S> A = A0;
   const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, SH::TY);
-  A.a_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8, step_latency(sizeof(S), EqOf<EQ>::coupled));
+  if (!ctx->step_chunk)
+    ctx->step_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8, step_latency(sizeof(S), EqOf<EQ>::coupled));
+  A.a_chunk = ctx->step_chunk;
   for (double &inv : A.inv) inv = lap_coef<2>(inv);  // the 13-point sum's 1/12
   step_coefs_f32(A);
   const dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
