@@ -175,10 +175,15 @@ static int launch_stage_t(cf_ctx *ctx, const StageArgs<S> &A0, cudaStream_t st) 
   StageArgs<S> A = A0;
   dim3 block(TX, TY);
   unsigned gx = ceil_div(A.N, TW), gy = ceil_div(A.N, TY);
-  // the plain right-hand side moves 4 words a site and marches shorter chunks (2 halo planes of
-  // phi each, from L2) to keep more CTAs in flight: 8 planes against 16, N = 256 117 -> 110 us, N =
-  // 200 80 -> 71 us; 32 planes 115 us
-  A.a_chunk = STAGE == 0 && A.N >= 64 ? 8 : pick_a_chunk(A.N, (int)(gx * gy));
+  // The plain right-hand side moves 4 words a site and marches shorter chunks (2 H halo planes
+  // of phi each, from L2) to keep more CTAs in flight.  Small lattices have too few CTAs for
+  // chunks of 8; the 13-point stencil, whose chunks re-read twice the planes, takes them
+  // earlier.  us with 4 / 8 / 16 planes, FRW 7-point: N = 80 8.7 / 10.4 / 14.3, 136 22.2 / 24.8, 152
+  // 33.0 / 32.0, 200 67.9 / 70 / 78, 256 111 / 109 / 116, 512 820 / 827 / 828; 13-point: 80 8.8 / 12.4
+  // / 16.5, 120 14.5 / 16.5, 136 26.3 / 25.8, 256 119 / 117 / 127, 512 917 / 910 / 913; comoving
+  // 7-point: 128 22.6 / 26.6 / 24.7, 152 56.3 / 55.2; 13-point: 104 16.5 / 20.7 / 20.7, 128 30.2 /
+  // 28.3 / 26.6, 256 203 / 196 / 193.
+  A.a_chunk = STAGE == 0 ? (A.N < (H == 2 ? 128 : 144) ? 4 : 8) : pick_a_chunk(A.N, (int)(gx * gy));
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, STAGE == 0 ? CF_PROF_OTHER : STAGE - 1, st);
   if (A.N % TW == 0 && A.N % TY == 0)
