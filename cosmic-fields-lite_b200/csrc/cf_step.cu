@@ -181,9 +181,10 @@ static int launch_stage_t(cf_ctx *ctx, const StageArgs<S> &A0, cudaStream_t st) 
   // earlier.  us with 4 / 8 / 16 planes, FRW 7-point: N = 80 8.7 / 10.4 / 14.3, 136 22.2 / 24.8, 152
   // 33.0 / 32.0, 200 67.9 / 70 / 78, 256 111 / 109 / 116, 512 820 / 827 / 828; 13-point: 80 8.8 / 12.4
   // / 16.5, 120 14.5 / 16.5, 136 26.3 / 25.8, 256 119 / 117 / 127, 512 917 / 910 / 913; comoving
-  // 7-point: 128 22.6 / 26.6 / 24.7, 152 56.3 / 55.2; 13-point: 104 16.5 / 20.7 / 20.7, 128 30.2 /
+  // 7-point (a curvature plane more): 128 22.6 / 26.6 / 24.7, 144 49.6 / 53.0, 152 56.3 / 55.2; 13-point: 104 16.5 / 20.7 / 20.7, 128 30.2 /
   // 28.3 / 26.6, 256 203 / 196 / 193.
-  A.a_chunk = STAGE == 0 ? (A.N < (H == 2 ? 128 : 144) ? 4 : 8) : pick_a_chunk(A.N, (int)(gx * gy));
+  constexpr int small = H == 2 ? 128 : (EqOf<EQ>::coupled ? 152 : 144);
+  A.a_chunk = STAGE == 0 ? (A.N < small ? 4 : 8) : pick_a_chunk(A.N, (int)(gx * gy));
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
   ProfScope ps(ctx, STAGE == 0 ? CF_PROF_OTHER : STAGE - 1, st);
   if (A.N % TW == 0 && A.N % TY == 0)
