@@ -28,8 +28,8 @@ enum EdKind : int { ED_QUAD = 0, ED_LAMBDA = 1, ED_SQRT = 2, ED_CURV = 3 };
 // `rowmax` (optional): receives the largest sum of rho^2 over 64 consecutive sites of a row
 // (fixed order, an integer max of the bit pattern): times N^2 ceil(N / 64) it bounds sum_x
 // rho^2, which Parseval turns into a bound on every spectrum bin.
-// MEAN: instead of rho, its mean over a (summed in increasing a, then divided by N) and its
-// slice at a = 0, each optional; one chunk of all planes.
+// MEAN: instead of rho, its mean over a (summed in increasing a, then divided by N; one chunk of
+// all planes) and its slice at a = 0, each optional.
 template <typename S>
 struct EnergyArgs {
   const S *x, *xlo, *psi;
@@ -134,13 +134,24 @@ __device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long t
   }
 }
 
-// Warp tasks of a lattice, and planes per warp: chunks of at most 32 (two planes more are read
-// per chunk), shorter while `lattices` of them give fewer than 16 warps per SM.
+// Warp tasks of a lattice (8 a CTA).
 inline long long energy_tasks(int N) { return (long long)N * ((N + ED_TILE - 1) / ED_TILE); }
 
-inline int energy_chunk(int N, int lattices) {
+// CTAs per SM: 64 registers for the forms with a polynomial potential, up to 80 for the others.
+constexpr int energy_per_sm(int ed) { return ed <= ED_LAMBDA ? 4 : 3; }
+
+// Planes per warp: chunks of at most 32 (two planes more are read per chunk), shorter while
+// `lattices` of them give fewer than 16 warps per SM.  Where the CTAs of such chunks make a wave and
+// a part of a second one, the chunk whose planes (and two more) times waves are least: us, FP64,
+// N = 200 FRW 55.6 -> 43.2, comoving 70.1 -> 59.3, N = 224 FRW 64.0 -> 55.6.
+inline int energy_chunk(int N, int lattices, int per_sm) {
   int ch = 32;
   while (ch > 2 && lattices * energy_tasks(N) * ((N + ch - 1) / ch) < 148LL * 16) ch /= 2;
+  const long long row = lattices * ((energy_tasks(N) + 7) / 8), slots = 148LL * per_sm;
+  auto waves = [&](int c) { return (row * ((N + c - 1) / c) + slots - 1) / slots; };
+  if (ch < 32 || waves(32) != 2) return ch;
+  for (int c : {24, 16, 12, 8})
+    if (waves(c) * (c + 2) < waves(ch) * (ch + 2)) ch = c;
   return ch;
 }
 

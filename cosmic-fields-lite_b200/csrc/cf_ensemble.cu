@@ -936,7 +936,7 @@ static int spectra(cf_ensemble *E, double t, double *d_out, cudaStream_t st) {
   }
   for (auto &c : E->classes) {
     const int n = (int)c.members.size();
-    const int ch = energy_chunk(c.N, n);
+    const int ch = energy_chunk(c.N, n, 3);
     const dim3 grid((unsigned)((energy_tasks(c.N) + 7) / 8), (unsigned)((c.N + ch - 1) / ch), n);
     if (E->word == 4)
       k_ens_energy<float><<<grid, 256, 0, st>>>(E->dm, c.d_members, c.rho, c.N, ch, a2);

@@ -23,12 +23,28 @@
 
 namespace cfb {
 
-template <typename S, int ED, bool MEAN>
+template <typename S, int ED>
 __global__ void __launch_bounds__(256) k_energy(const EnergyArgs<S> A) {
   const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (task >= (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE)) return;  // whole warps
   const int a0 = blockIdx.y * A.a_chunk;
-  energy_march<S, ED, MEAN>(A, task, a0, min(a0 + A.a_chunk, A.N));
+  energy_march<S, ED, false>(A, task, a0, min(a0 + A.a_chunk, A.N));
+}
+
+// The mean over a (and the slice at a = 0): one warp sums a column of 64 sites, so there are few
+// warps, each with more loads in flight at 3 CTAs per SM (72 to 80 registers) than at 4.
+template <typename S, int ED, int PER_SM>
+__global__ void __launch_bounds__(256, PER_SM) k_energy_mean(const EnergyArgs<S> A) {
+  const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
+  if (task >= (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE)) return;
+  const int a0 = blockIdx.y * A.a_chunk;  // 0
+  energy_march<S, ED, true>(A, task, a0, min(a0 + A.a_chunk, A.N));
+}
+// 4 CTAs per SM where that makes one wave of what 3 would need two for (N = 512, FP32 comoving 0.95
+// -> 0.72 ms).
+static int mean_per_sm(int N) {
+  const long long n = (energy_tasks(N) + 7) / 8;
+  return n > 148 * 3 && n <= 148 * 4 ? 4 : 3;
 }
 
 // d rho / dt of the FRW Klein-Gordon equation (src/equations_cuda.cu:372-424):
@@ -499,7 +515,7 @@ int mode_power_spectrum_s2(cf_ctx *ctx, const void *d_state, double a_t, double 
   return bin_spectrum(ctx, true, a_t, d_out, st, bound);
 }
 
-// What the energy passes write: rho (with rowmax optional), or its mean and slice.
+// What the energy passes write: rho (with rowmax optional), or its mean over a and its slice.
 struct EnergyOut {
   double *rho = nullptr;
   unsigned long long *rowmax = nullptr;
@@ -507,28 +523,33 @@ struct EnergyOut {
 };
 
 template <typename S, int ED>
-static void launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
-                          double q, cudaStream_t st) {
+static int launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
+                         double q, cudaStream_t st) {
   const long long N3 = ctx->N3;
   const int N = (int)ctx->N;
   const S *x = (const S *)d_state;
   EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * N3 : x, (const S *)psi, o.rho, o.slice, o.mean, N, N, m2, inv, q, o.rowmax};
   const unsigned gx = (unsigned)((energy_tasks(N) + 7) / 8);
-  if (!o.rho) {
-    k_energy<S, ED, true><<<gx, 256, 0, st>>>(A);
-  } else {
-    A.a_chunk = energy_chunk(N, 1);
-    k_energy<S, ED, false><<<dim3(gx, (unsigned)((N + A.a_chunk - 1) / A.a_chunk)), 256, 0, st>>>(A);
+  if (o.rho) {
+    A.a_chunk = energy_chunk(N, 1, energy_per_sm(ED));
+    k_energy<S, ED><<<dim3(gx, (unsigned)((N + A.a_chunk - 1) / A.a_chunk)), 256, 0, st>>>(A);
+    CF_LAUNCHED(ctx);
+    return CF_OK;
   }
+  A.a_chunk = o.mean ? N : 1;  // the slice alone takes the first plane
+  if (mean_per_sm(N) == 4)
+    k_energy_mean<S, ED, 4><<<gx, 256, 0, st>>>(A);
+  else
+    k_energy_mean<S, ED, 3><<<gx, 256, 0, st>>>(A);
+  CF_LAUNCHED(ctx);
+  return CF_OK;
 }
 
 template <int ED>
-static void launch_energy_p(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
-                            double q, cudaStream_t st) {
-  if (ctx->p.precision == CF_FP32_COMP)
-    launch_energy<float, ED>(ctx, d_state, psi, o, m2, inv, q, st);
-  else
-    launch_energy<double, ED>(ctx, d_state, psi, o, m2, inv, q, st);
+static int launch_energy_p(cf_ctx *ctx, const void *d_state, const void *psi, const EnergyOut &o, double m2, double inv,
+                           double q, cudaStream_t st) {
+  if (ctx->p.precision == CF_FP32_COMP) return launch_energy<float, ED>(ctx, d_state, psi, o, m2, inv, q, st);
+  return launch_energy<double, ED>(ctx, d_state, psi, o, m2, inv, q, st);
 }
 
 static int energy_density_b(cf_ctx *ctx, const void *d_state, double t, const EnergyOut &o, cudaStream_t st) {
@@ -542,16 +563,11 @@ static int energy_density_b(cf_ctx *ctx, const void *d_state, double t, const En
   if (eq == CF_EQ_COMOVING_FRW || eq == CF_EQ_APPROX_COMOVING_FRW) CF_TRY(psi_at(ctx, t, st, &ps, &dps));
   if (eq == CF_EQ_FIXED_CURVATURE_FRW) ps = ctx->fixed_e2m1;
   ProfScope prof(ctx, CF_PROF_SPECTRUM, st);
-  if (ps)
-    launch_energy_p<ED_CURV>(ctx, d_state, ps, o, m2, inv, 0.0, st);
-  else if (eq == CF_EQ_LAMBDA_FRW)
-    launch_energy_p<ED_LAMBDA>(ctx, d_state, nullptr, o, m2, inv, ctx->p.lambda, st);
-  else if (eq == CF_EQ_SQRT_FRW)
-    launch_energy_p<ED_SQRT>(ctx, d_state, nullptr, o, m2, inv, 1.0 / (ctx->p.f_a * ctx->p.f_a), st);
-  else
-    launch_energy_p<ED_QUAD>(ctx, d_state, nullptr, o, m2, inv, 0.0, st);
-  CF_LAUNCHED(ctx);
-  return CF_OK;
+  if (ps) return launch_energy_p<ED_CURV>(ctx, d_state, ps, o, m2, inv, 0.0, st);
+  if (eq == CF_EQ_LAMBDA_FRW) return launch_energy_p<ED_LAMBDA>(ctx, d_state, nullptr, o, m2, inv, ctx->p.lambda, st);
+  if (eq == CF_EQ_SQRT_FRW)
+    return launch_energy_p<ED_SQRT>(ctx, d_state, nullptr, o, m2, inv, 1.0 / (ctx->p.f_a * ctx->p.f_a), st);
+  return launch_energy_p<ED_QUAD>(ctx, d_state, nullptr, o, m2, inv, 0.0, st);
 }
 
 int energy_density(cf_ctx *ctx, const void *d_state, double t, double *d_rho, cudaStream_t st) {
@@ -587,27 +603,32 @@ __global__ void k_axis_mean(const double *__restrict__ f, double *__restrict__ o
   }
 }
 
+// Whether the mean over a is summed by the energy pass itself, each warp marching over all planes
+// (the sum's order is fixed, so a column is one warp's), and no density is written: where its
+// CTAs fill enough of the waves they make.  us, one march / the density and a pass over it: FP64 FRW N
+// = 288 (41% of a wave) 180 / 165, 320 (45%) 194 / 203, 384 (65%) 240 / 317, 448 (88%) 297 / 488,
+// 576 (73% of two) 761 / 1081; FP32 comoving 320 289 / 270, 336 (57%) 309 / 325, 384 356 / 427; FP32 sqrt 336
+// 342 / 342.
+static bool slices_in_one_march(const cf_ctx *ctx) {
+  const long long n = (energy_tasks((int)ctx->N) + 7) / 8, slots = 148LL * mean_per_sm((int)ctx->N);
+  const double filled = (double)n / (double)((n + slots - 1) / slots * slots);
+  return filled >= (ctx->word == 8 ? 0.45 : 0.56);
+}
+
 int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, double *d_avg, cudaStream_t st) {
+  EnergyOut o;
+  o.slice = d_slice;
+  o.mean = d_avg;
+  if (!d_slice && !d_avg) return CF_OK;
+  if (!d_avg || slices_in_one_march(ctx)) return energy_density_b(ctx, d_state, t, o, st);
   const long long NN = ctx->N * ctx->N;
-  // With a warp per SM sub-partition or more from one chunk of all planes, the energy pass
-  // sums over a itself and the density is not written; smaller lattices need the chunks
-  // (N = 512: 0.96 ms against 1.30 for the density and a pass over it).
-  if (energy_tasks((int)ctx->N) >= 148LL * 8) {
-    EnergyOut o;
-    o.slice = d_slice;
-    o.mean = d_avg;
-    if (!d_slice && !d_avg) return CF_OK;
-    return energy_density_b(ctx, d_state, t, o, st);
-  }
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
   CF_TRY(energy_density(ctx, d_state, t, ctx->spec_field, st));
   if (d_slice)
     CF_TRY_CUDA(cudaMemcpyAsync(d_slice, ctx->spec_field, NN * sizeof(double), cudaMemcpyDeviceToDevice, st));
-  if (d_avg) {
-    ProfScope ps(ctx, CF_PROF_SPECTRUM, st);
-    k_axis_mean<<<grid_for(NN), 256, 0, st>>>(ctx->spec_field, d_avg, NN, (int)ctx->N);
-    CF_LAUNCHED(ctx);
-  }
+  ProfScope ps(ctx, CF_PROF_SPECTRUM, st);
+  k_axis_mean<<<grid_for(NN), 256, 0, st>>>(ctx->spec_field, d_avg, NN, (int)ctx->N);
+  CF_LAUNCHED(ctx);
   return CF_OK;
 }
 
