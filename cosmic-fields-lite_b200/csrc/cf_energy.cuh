@@ -137,19 +137,20 @@ __device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long t
 // Warp tasks of a lattice (8 a CTA).
 inline long long energy_tasks(int N) { return (long long)N * ((N + ED_TILE - 1) / ED_TILE); }
 
-// CTAs per SM: 64 registers for the forms with a polynomial potential, up to 80 for the others.
-constexpr int energy_per_sm(int ed) { return ed <= ED_LAMBDA ? 4 : 3; }
+// CTAs per SM: 64 registers for the forms with a polynomial potential and, by its launch bound, the
+// FP64 sqrt potential; up to 80 for the others.
+constexpr int energy_per_sm(int ed, size_t word) { return ed <= ED_LAMBDA || (ed == ED_SQRT && word == 8) ? 4 : 3; }
 
 // Planes per warp: chunks of at most 32 (two planes more are read per chunk), shorter while
-// `lattices` of them give fewer than 16 warps per SM.  Where the CTAs of such chunks make a wave and
-// a part of a second one, the chunk whose planes (and two more) times waves are least: us, FP64,
-// N = 200 FRW 55.6 -> 43.2, comoving 70.1 -> 59.3, N = 224 FRW 64.0 -> 55.6.
+// `lattices` of them give fewer than 16 warps per SM.  Where the CTAs of such chunks make at most
+// two waves, the chunk whose planes (and two more) times waves are least: us, FP64, N = 160 FRW
+// 28.6 -> 23.0, N = 200 FRW 55.6 -> 43.2, comoving 70.1 -> 59.3, N = 224 FRW 64.0 -> 55.6.
 inline int energy_chunk(int N, int lattices, int per_sm) {
   int ch = 32;
   while (ch > 2 && lattices * energy_tasks(N) * ((N + ch - 1) / ch) < 148LL * 16) ch /= 2;
   const long long row = lattices * ((energy_tasks(N) + 7) / 8), slots = 148LL * per_sm;
   auto waves = [&](int c) { return (row * ((N + c - 1) / c) + slots - 1) / slots; };
-  if (ch < 32 || waves(32) != 2) return ch;
+  if (ch < 32 || waves(32) > 2) return ch;
   for (int c : {24, 16, 12, 8})
     if (waves(c) * (c + 2) < waves(ch) * (ch + 2)) ch = c;
   return ch;

@@ -23,8 +23,10 @@
 
 namespace cfb {
 
+// The FP64 sqrt potential is held to 64 registers (4 CTAs per SM, 24 bytes spilled): N = 256 111 -> 89
+// us, N = 512 751 -> 646; the other forms have what they need (0: no bound).
 template <typename S, int ED>
-__global__ void __launch_bounds__(256) k_energy(const EnergyArgs<S> A) {
+__global__ void __launch_bounds__(256, ED == ED_SQRT && sizeof(S) == 8 ? 4 : 0) k_energy(const EnergyArgs<S> A) {
   const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   if (task >= (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE)) return;  // whole warps
   const int a0 = blockIdx.y * A.a_chunk;
@@ -531,7 +533,7 @@ static int launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, cons
   EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * N3 : x, (const S *)psi, o.rho, o.slice, o.mean, N, N, m2, inv, q, o.rowmax};
   const unsigned gx = (unsigned)((energy_tasks(N) + 7) / 8);
   if (o.rho) {
-    A.a_chunk = energy_chunk(N, 1, energy_per_sm(ED));
+    A.a_chunk = energy_chunk(N, 1, energy_per_sm(ED, sizeof(S)));
     k_energy<S, ED><<<dim3(gx, (unsigned)((N + A.a_chunk - 1) / A.a_chunk)), 256, 0, st>>>(A);
     CF_LAUNCHED(ctx);
     return CF_OK;
