@@ -25,9 +25,8 @@ enum EdKind : int { ED_QUAD = 0, ED_LAMBDA = 1, ED_SQRT = 2, ED_CURV = 3 };
 // of the other warps.  With a row per block and every stencil point loaded and widened on
 // its own the pass waited on memory at a third of the bandwidth: N = 512 FP32_COMP comoving
 // 1.14 -> 0.84 ms (28 bytes per site: 0.58 at the copy rate).
-// `rowmax` (optional): receives the largest sum of rho^2 over 64 consecutive sites of a row
-// (fixed order, an integer max of the bit pattern): times N^2 ceil(N / 64) it bounds sum_x
-// rho^2, which Parseval turns into a bound on every spectrum bin.
+// SQUARES: returns the lane's sum of rho^2 over its sites (in increasing a): the
+// lattice's sum, by Parseval N^-3 times that of the spectrum, scales the binning (cf_spectrum.cu).
 // MEAN: instead of rho, its mean over a (summed in increasing a, then divided by N; one chunk of
 // all planes) and its slice at a = 0, each optional.
 template <typename S>
@@ -37,13 +36,15 @@ struct EnergyArgs {
   double *slice, *mean;
   int N, a_chunk;
   double m2, inv, q;
-  unsigned long long *rowmax;
 };
 constexpr int ED_TILE = 64;
 
-template <typename S, int ED, bool MEAN>
-__device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long task, int a0, int a1) {
+template <typename S, int ED, bool MEAN, bool SQUARES = false>
+__device__ __forceinline__ double energy_march(const EnergyArgs<S> &A, long long task, int a0, int a1) {
   using V2 = typename VecOf<S, 2>::T;
+  // Two planes a turn, whose loads the compiler interleaves only for the mean: for rho that takes 78
+  // registers and a CTA of the SM (N = 512 559 -> 646 us), with the squares also where it may not.
+  constexpr int U = SQUARES ? 1 : 2;
   const int N = A.N, lane = threadIdx.x & 31;
   const long long NN = (long long)N * N, N3 = NN * N;
   const int b = (int)(task % N), c0 = (int)(task / N) * ED_TILE;
@@ -72,9 +73,9 @@ __device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long t
   };
   double2 prev = pair(A.x, A.xlo, NN * (a0 == 0 ? N - 1 : a0 - 1) + row), cur = pair(A.x, A.xlo, NN * a0 + row);
   const bool vec = (reinterpret_cast<unsigned long long>(A.rho) & 15) == 0;  // a caller's rho may be 8-byte aligned
-  double most = 0.0;
+  double ss = 0.0;
   double2 sum = make_double2(0.0, 0.0);
-#pragma unroll 2
+#pragma unroll U
   for (int a = a0; a < a1; ++a) {
     const long long pl = NN * a;
     const double2 next = pair(A.x, A.xlo, NN * (a + 1 == N ? 0 : a + 1) + row);
@@ -118,20 +119,15 @@ __device__ __forceinline__ void energy_march(const EnergyArgs<S> &A, long long t
         else
           o[0] = r.x, o[1] = r.y;
       }
-      if (A.rowmax) {
-        double ss = act ? r.x * r.x + r.y * r.y : 0.0;
-        for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
-        most = fmax(most, ss);
-      }
+      if (SQUARES && act) ss += r.x * r.x + r.y * r.y;
     }
+    if constexpr (!MEAN && !SQUARES) asm volatile("" ::: "memory");
     prev = cur, cur = next;
   }
   if constexpr (MEAN) {
     if (act && A.mean) A.mean[row] = sum.x / (double)N, A.mean[row + 1] = sum.y / (double)N;
-  } else {
-    // non-negative doubles order like their bit patterns
-    if (A.rowmax && lane == 0) atomicMax(A.rowmax, (unsigned long long)__double_as_longlong(most));
   }
+  return ss;
 }
 
 // Warp tasks of a lattice (8 a CTA).

@@ -445,7 +445,7 @@ __global__ void __launch_bounds__(256) k_ens_energy(const EnsMember *members, co
   const EnsMember mb = members[class_members[blockIdx.z]];
   const S *x = (const S *)mb.x;
   EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * mb.N3 : x, nullptr, rho + (long long)blockIdx.z * mb.N3, nullptr, nullptr,
-                  N, a_chunk, mb.m2, mb.inv_scale / a2, 0.0, nullptr};
+                  N, a_chunk, mb.m2, mb.inv_scale / a2, 0.0};
   const int a0 = blockIdx.y * a_chunk;
   energy_march<S, ED_QUAD, false>(A, task, a0, min(a0 + a_chunk, N));
 }

@@ -175,7 +175,7 @@ struct cf_ctx {
   double *small = nullptr;
   size_t small_n = 0;
   unsigned long long *bins = nullptr;   // 2 * s2_bins words: (lo, hi) fixed point
-  unsigned long long *maxbits = nullptr;
+  unsigned long long *maxbits = nullptr;  // the scale's maximum or sum; a count of CTAs (grid_sum)
   long long spec_mult = 0;  // scale multiplier of the last binning (bin_spectrum)
   // Host <-> device transfers of an FP32_COMP state (cf_state_upload / download):
   // two FP64 chunks used in turn, and the event that ends the last transfer.

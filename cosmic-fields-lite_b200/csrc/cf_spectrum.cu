@@ -5,8 +5,8 @@
 // :25).  Here every mode value is converted to a 128-bit fixed-point integer
 // whose scale is a power of two chosen from an order-independent upper bound on
 // any bin -- the largest mode value times the entry count (a max pass over the
-// modes), or by Parseval a sum over the lattice that an earlier pass forms: of rho^2
-// in the energy pass for the density spectrum, of the state in the widening of an FP32_COMP
+// modes), or by Parseval a sum over the lattice that an earlier pass forms in a fixed order: of
+// rho^2 in the energy pass for the density spectrum, of the state in the widening of an FP32_COMP
 // state for the mode spectrum -- and the bins accumulate those
 // integers with 64-bit integer atomics (carry propagated to the high word).
 // Integer addition is associative, so the bins are bit-reproducible, and the
@@ -16,6 +16,7 @@
 #include <cuda_runtime.h>
 #include <cufft.h>
 
+#include <algorithm>
 #include <cmath>
 
 #include "cf_energy.cuh"
@@ -23,14 +24,52 @@
 
 namespace cfb {
 
-// The FP64 sqrt potential is held to 64 registers (4 CTAs per SM, 24 bytes spilled): N = 256 111 -> 89
-// us, N = 512 751 -> 646; the other forms have what they need (0: no bound).
-template <typename S, int ED>
-__global__ void __launch_bounds__(256, ED == ED_SQRT && sizeof(S) == 8 ? 4 : 0) k_energy(const EnergyArgs<S> A) {
+// The sum over a CTA of 256 threads, in a fixed order; thread 0 has it.
+__device__ __forceinline__ double cta_sum(double v) {
+  __shared__ double w[8];
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+  if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = v;
+  __syncthreads();
+  double t = w[0];
+  for (int k = 1; k < 8; ++k) t += w[k];
+  return t;
+}
+
+// The sum of v over a grid of CTAs of 256 threads, in a fixed order, as a bit pattern in B.total: each
+// CTA leaves its sum, and the one that arrives last adds them (the count wraps to 0 by itself).
+struct GridSum {
+  double *part;               // a word per CTA
+  unsigned *arrived;          // 0 between grids
+  unsigned long long *total;
+};
+__device__ __forceinline__ void grid_sum(const GridSum &B, double v, unsigned cta, unsigned ctas) {
+  __shared__ bool last;
+  const double t = cta_sum(v);
+  if (threadIdx.x == 0) {
+    B.part[cta] = t;
+    __threadfence();
+    last = atomicInc(B.arrived, ctas - 1) == ctas - 1;
+  }
+  __syncthreads();
+  if (!last) return;
+  __threadfence();
+  double s = 0.0;
+  for (unsigned i = threadIdx.x; i < ctas; i += 256) s += __ldcg(B.part + i);
+  s = cta_sum(s);
+  if (threadIdx.x == 0) *B.total = (unsigned long long)__double_as_longlong(s);
+}
+
+// The FP64 sqrt potential is held to 64 registers (4 CTAs per SM, 8 bytes spilled): N = 256 111 -> 89
+// us, N = 512 751 -> 651.
+template <typename S, int ED, bool SQUARES>
+__global__ void __launch_bounds__(256, energy_per_sm(ED, sizeof(S)))
+    k_energy(const EnergyArgs<S> A, const GridSum B) {
   const long long task = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  if (task >= (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE)) return;  // whole warps
   const int a0 = blockIdx.y * A.a_chunk;
-  energy_march<S, ED, false>(A, task, a0, min(a0 + A.a_chunk, A.N));
+  double ss = 0.0;
+  if (task < (long long)A.N * ((A.N + ED_TILE - 1) / ED_TILE))  // whole warps
+    ss = energy_march<S, ED, false, SQUARES>(A, task, a0, min(a0 + A.a_chunk, A.N));
+  if constexpr (SQUARES) grid_sum(B, ss, blockIdx.y * gridDim.x + blockIdx.x, gridDim.x * gridDim.y);
 }
 
 // The mean over a (and the slice at a = 0): one warp sums a column of 64 sites, so there are few
@@ -96,14 +135,11 @@ __global__ void k_export_f32(const float *__restrict__ s, double *__restrict__ o
     out[i] = (double)s[i] + (double)s[n2 + i];
 }
 
-// The same for the mode spectrum, with the largest block's sum of phi^2 + pi^2 / m^2 (fixed order,
-// an integer max of the bit pattern) in *blockmax: times the number of blocks it bounds the sum
-// over the lattice, and by Parseval, N^3 times that, the sum of the weighted mode values
-// |phi_k|^2 + |pi_k|^2 / (m^2 + k^2 / a^2), so the binning needs no pass over the modes to find
-// their maximum.
+// The same for the mode spectrum, with the sum of phi^2 + pi^2 / m^2: by Parseval N^3 times
+// it bounds the sum of the weighted mode values |phi_k|^2 + |pi_k|^2 / (m^2 + k^2 / a^2),
+// so the binning needs no pass over the modes to find their maximum.
 __global__ void __launch_bounds__(256) k_export_bound_f32(const float *__restrict__ s, double *__restrict__ out,
-                                                          long long n2, double inv_m2,
-                                                          unsigned long long *__restrict__ blockmax) {
+                                                          long long n2, double inv_m2, const GridSum B) {
   const long long stride = 2LL * gridDim.x * blockDim.x;
   double ss = 0.0;
   for (long long i = 2 * ((long long)blockIdx.x * blockDim.x + threadIdx.x); i < n2; i += stride) {
@@ -113,15 +149,7 @@ __global__ void __launch_bounds__(256) k_export_bound_f32(const float *__restric
     const double q = v.x * v.x + v.y * v.y;
     ss += 2 * i < n2 ? q : q * inv_m2;
   }
-  __shared__ double part[8];
-  for (int o = 16; o > 0; o >>= 1) ss += __shfl_down_sync(0xffffffffu, ss, o);
-  if ((threadIdx.x & 31) == 0) part[threadIdx.x >> 5] = ss;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    double t = part[0];
-    for (int w = 1; w < 8; ++w) t += part[w];
-    atomicMax(blockmax, (unsigned long long)__double_as_longlong(t));
-  }
+  grid_sum(B, ss, blockIdx.x, gridDim.x);
 }
 
 // FP64 [phi | pi] -> FP32_COMP state.
@@ -251,10 +279,11 @@ __global__ void __launch_bounds__(256) k_spec_max(SpecIn A, long long hc_count, 
   if ((threadIdx.x & 31) == 0) atomicMax(maxbits + blockIdx.y, (unsigned long long)__double_as_longlong(m));
 }
 
-// Power-of-two exponent e with (max * entries) * 2^e <= 2^126.
+// Power-of-two exponent e with (m * pairs) * 2^e <= 2^126, m the largest mode value or a sum that
+// bounds them (a rounded one: the two bits above leave room); 0 without a finite one.
 __device__ __forceinline__ int fixed_exponent(unsigned long long maxbits, long long pairs) {
   const double m = __longlong_as_double((long long)maxbits);
-  if (!(m > 0.0)) return 0;
+  if (!(m > 0.0) || isinf(m)) return 0;
   int ex;
   frexp(m * (double)pairs, &ex);  // m*pairs < 2^ex
   return 126 - ex;
@@ -415,7 +444,7 @@ int ensure_spectrum_scratch(cf_ctx *ctx, int nfields) {
       return CF_ERR_NOMEM;
     }
     if (cudaMalloc(&ctx->bins, 2 * (size_t)ctx->s2_bins * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&ctx->maxbits, sizeof(unsigned long long)) != cudaSuccess ||
+        cudaMalloc(&ctx->maxbits, 2 * sizeof(unsigned long long)) != cudaSuccess ||
         cudaMalloc(&ctx->s2_counts, (size_t)ctx->s2_bins * sizeof(int64_t)) != cudaSuccess) {
       set_error("cudaMalloc spectrum bins failed");
       return CF_ERR_NOMEM;
@@ -424,7 +453,7 @@ int ensure_spectrum_scratch(cf_ctx *ctx, int nfields) {
     k_s2_counts<<<orbit_blocks((int)ctx->N), 256>>>((int)ctx->N, (unsigned long long *)ctx->s2_counts);
     CF_LAUNCHED(ctx);
     CF_TRY_CUDA(cudaMemset(ctx->bins, 0, 2 * (size_t)ctx->s2_bins * sizeof(unsigned long long)));
-    CF_TRY_CUDA(cudaMemset(ctx->maxbits, 0, sizeof(unsigned long long)));
+    CF_TRY_CUDA(cudaMemset(ctx->maxbits, 0, 2 * sizeof(unsigned long long)));
     CF_TRY_CUDA(cudaDeviceSynchronize());
   }
   const int N = (int)ctx->N;
@@ -487,6 +516,13 @@ int power_spectrum_s2(cf_ctx *ctx, const double *d_f, double *d_out, cudaStream_
   return bin_spectrum(ctx, false, 1.0, d_out, st);
 }
 
+// The sum a bound comes from, into ctx->maxbits.  The CTAs' words are the bins, which the binning clears
+// afterwards (2 s2_bins = 1.5 N^2 + 2 words; k_energy makes at most N^2 / 8 CTAs for N <= 64, max(4736,
+// N^3 / 2048) beyond, the widening at most min(592, N^3 / 256)).
+static GridSum grid_sum_of(cf_ctx *ctx) {
+  return GridSum{(double *)ctx->bins, (unsigned *)(ctx->maxbits + 1), ctx->maxbits};
+}
+
 int mode_power_spectrum_s2(cf_ctx *ctx, const void *d_state, double a_t, double *d_out, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 2));
   const double *x = (const double *)d_state;
@@ -494,15 +530,16 @@ int mode_power_spectrum_s2(cf_ctx *ctx, const void *d_state, double a_t, double 
   if (ctx->p.precision != CF_FP64) {
     // The state is widened for the transform anyway, so its sums come along and bound the bins
     // (N = 512: the 0.49 ms of the max pass) unless the bound could be more than 2^20 above the
-    // sum of the mode values (k_max^2 against a^2 m^2): the fixed point keeps 2^-106 of that
-    // sum, more than the FP64 results resolve.  An FP64 state would need a pass of its own.
+    // sum of the mode values (k_max^2 against a^2 m^2).  The fixed point then keeps 2^-106 of that sum
+    // at least, the max pass (largest value times entry count) 2^-100 at N = 512.  An FP64 state
+    // would need a pass of its own.
     const long long n2 = 2 * ctx->N3;
     const double m2 = ctx->p.m * ctx->p.m, k = 3.14159265358979323846 * ctx->N / ctx->p.L;
-    const unsigned blocks = grid_for(n2 / 2);
     if (3.0 * k * k < 1048576.0 * m2 * a_t * a_t) {
-      bound = ctx->N3 * (long long)blocks;
-      CF_TRY_CUDA(cudaMemsetAsync(ctx->maxbits, 0, sizeof(unsigned long long), st));
-      k_export_bound_f32<<<blocks, 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2, 1.0 / m2, ctx->maxbits);
+      bound = ctx->N3;
+      // 4 CTAs per SM: more of them queue for the count (N = 128, us per spectrum 107 with 4736, 102 with 592)
+      k_export_bound_f32<<<std::min(grid_for(n2 / 2), 148u * 4), 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2,
+                                                                              1.0 / m2, grid_sum_of(ctx));
     } else {
       k_export_f32<<<grid_for(n2), 256, 0, st>>>((const float *)d_state, ctx->spec_field, n2);
     }
@@ -517,10 +554,11 @@ int mode_power_spectrum_s2(cf_ctx *ctx, const void *d_state, double a_t, double 
   return bin_spectrum(ctx, true, a_t, d_out, st, bound);
 }
 
-// What the energy passes write: rho (with rowmax optional), or its mean over a and its slice.
+// What the energy passes write: rho (and, optional, the sum of its squares), or its mean over a and
+// its slice.
 struct EnergyOut {
   double *rho = nullptr;
-  unsigned long long *rowmax = nullptr;
+  bool squares = false;  // the sum of rho^2 as well (grid_sum_of)
   double *slice = nullptr, *mean = nullptr;
 };
 
@@ -530,11 +568,15 @@ static int launch_energy(cf_ctx *ctx, const void *d_state, const void *psi, cons
   const long long N3 = ctx->N3;
   const int N = (int)ctx->N;
   const S *x = (const S *)d_state;
-  EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * N3 : x, (const S *)psi, o.rho, o.slice, o.mean, N, N, m2, inv, q, o.rowmax};
+  EnergyArgs<S> A{x, sizeof(S) == 4 ? x + 2 * N3 : x, (const S *)psi, o.rho, o.slice, o.mean, N, N, m2, inv, q};
   const unsigned gx = (unsigned)((energy_tasks(N) + 7) / 8);
   if (o.rho) {
     A.a_chunk = energy_chunk(N, 1, energy_per_sm(ED, sizeof(S)));
-    k_energy<S, ED><<<dim3(gx, (unsigned)((N + A.a_chunk - 1) / A.a_chunk)), 256, 0, st>>>(A);
+    const unsigned chunks = (unsigned)((N + A.a_chunk - 1) / A.a_chunk);
+    if (o.squares)
+      k_energy<S, ED, true><<<dim3(gx, chunks), 256, 0, st>>>(A, grid_sum_of(ctx));
+    else
+      k_energy<S, ED, false><<<dim3(gx, chunks), 256, 0, st>>>(A, GridSum{});
     CF_LAUNCHED(ctx);
     return CF_OK;
   }
@@ -635,22 +677,20 @@ int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, 
 }
 
 // The fixed-point scale comes from the energy pass: by Parseval the weighted HC
-// values of rho sum to N^3 sum_x rho^2 <= N^5 ceil(N/64) times the largest sum over 64
-// sites of a row, so no bin can exceed that bound, and the binning needs no pass of its own to find a maximum.
+// values of rho sum to N^3 sum_x rho^2, so no bin can exceed that, and the binning needs no
+// pass of its own to find a maximum.
 int density_spectrum_s2(cf_ctx *ctx, const void *d_state, double t, double *d_out, cudaStream_t st) {
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
-  CF_TRY_CUDA(cudaMemsetAsync(ctx->maxbits, 0, sizeof(unsigned long long), st));
   EnergyOut o;
   o.rho = ctx->spec_field;
-  o.rowmax = ctx->maxbits;
+  o.squares = true;
   CF_TRY(energy_density_b(ctx, d_state, t, o, st));
   CF_TRY_CUFFT(cufftSetStream(ctx->plan_d2z1, st));
   {
     ProfScope ps(ctx, CF_PROF_SPECTRUM, st);
     CF_TRY_CUFFT(cufftExecD2Z(ctx->plan_d2z1, (cufftDoubleReal *)ctx->spec_field, (cufftDoubleComplex *)ctx->spec_hc));
   }
-  const long long N = ctx->N;
-  return bin_spectrum(ctx, false, 1.0, d_out, st, N * N * N * N * N * ((N + ED_TILE - 1) / ED_TILE));
+  return bin_spectrum(ctx, false, 1.0, d_out, st, ctx->N3);
 }
 
 int s2_to_shells(cf_ctx *ctx, double *d_shells, int64_t *d_counts, cudaStream_t st) {
