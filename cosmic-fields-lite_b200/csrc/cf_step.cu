@@ -536,14 +536,22 @@ static int launch_step13_k(cf_ctx *ctx, const StepArgs<S> &A, dim3 grid, cudaStr
 }
 
 template <typename S, int EQ>
+static int step13_chunk(cf_ctx *ctx) {
+  using SH = Step13Shape<S, EQ>;
+  const int N = (int)ctx->N;
+  if (!ctx->step_chunk)
+    ctx->step_chunk = step_a_chunk(N, (int)(ceil_div(N, Step13Smem<S, SH::TX, SH::TY>::TW) * ceil_div(N, SH::TY)), SH::MB, 8,
+                                   step_latency(sizeof(S), EqOf<EQ>::coupled));
+  return ctx->step_chunk;
+}
+
+template <typename S, int EQ>
 static int launch_step13_t(cf_ctx *ctx, const StepArgs<S> &A0, cudaStream_t st) {
   using SH = Step13Shape<S, EQ>;
   using SM = Step13Smem<S, SH::TX, SH::TY>;
   StepArgs<S> A = A0;
   const unsigned gx = ceil_div(A.N, SM::TW), gy = ceil_div(A.N, SH::TY);
-  if (!ctx->step_chunk)
-    ctx->step_chunk = step_a_chunk(A.N, (int)(gx * gy), SH::MB, 8, step_latency(sizeof(S), EqOf<EQ>::coupled));
-  A.a_chunk = ctx->step_chunk;
+  A.a_chunk = step13_chunk<S, EQ>(ctx);
   for (double &inv : A.inv) inv = lap_coef<2>(inv);  // the 13-point sum's 1/12
   step_coefs_f32(A);
   const dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
@@ -776,20 +784,26 @@ int rk4_step_buffers(cf_ctx *ctx, void *d_state, void *acc, void *ya, void *yb, 
   return rk4_step_buffers_t<double>(ctx, d_state, acc, ya, yb, t, dt, st);
 }
 
-// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).  From N =
-// 72 to 120 the FP32 13-point comoving pass, whose CTAs take an SM each, leaves the Psi
-// refreshes beside it no room, and a march of its few planes costs as much as two of the
-// paired passes': 10 steps in one call, us per step paired / whole, N = 80 96 / 106, 96 108 /
-// 111, 112 151 / 161, 120 174 / 183, but 128 95 / 86 and 144 263 / 240; at 48 and 64 launches
-// bound both (75 / 75, 52 / 52) and one step per call is faster whole (91 / 86, 78 / 74).  Fixed Psi, which
-// refreshes nothing, loses only at 88 and 96, where the paired passes' grids are still one
-// wave and the whole pass has two 64-wide tiles per row: 80 25.2 / 23.6, 88 25.5 / 27.8, 96 26.6 /
-// 27.6, 104 40.9 / 33.9.
-static bool whole_step_route(const cf_ctx *ctx) {
+// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).  The FP32 13-point
+// pass with a curvature input has one CTA per SM, and the paired passes remain where that costs more
+// than the traffic they add (us per step, whole / paired):
+//   - comoving with the next step's Psi refreshes beside the step (psi_pipelined), which the pass
+//     leaves no room: N = 40 57 / 53, 48 66 / 60, 72 78 / 73, 96 108 / 103, 120 161 / 155.  From N = 128 the pass
+//     gains more than it delays them: 128 85 / 89, 136 238 / 254, 160 223 / 272;
+//   - else, where one wave takes all CTAs of a paired pass, which then march 4 planes, and the whole
+//     pass marches more than 6 (and 8 halo planes): fixed Psi N = 80 (6) 22.6 / 22.7, 88 (8) 26.7 / 23.7,
+//     96 (8) 26.0 / 25.4, 104 (two paired waves) 32.9 / 39.9; one comoving step per call 72 99 / 101,
+//     88 118 / 114, 96 129 / 123, 120 179 / 184; approximate 96 72 / 70.
+static bool whole_step_route(cf_ctx *ctx, int64_t nsteps) {
   if (ctx->p.flags & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS)) return false;
-  if (ctx->p.stencil != 13 || ctx->p.precision != CF_FP32_COMP) return true;
-  const int eq = shape_of(ctx->p.equation);
-  return !((eq == EQ_COMOV && ctx->N > 64 && ctx->N < 128) || (eq == EQ_FIXED && ctx->N > 80 && ctx->N <= 96));
+  const int eq = shape_of(ctx->p.equation), N = (int)ctx->N;
+  const bool coupled = eq == EQ_COMOV || eq == EQ_FIXED || eq == EQ_APPROX;
+  if (ctx->p.stencil != 13 || ctx->p.precision != CF_FP32_COMP || !coupled) return true;
+  if (psi_pipelined(ctx, nsteps) && N < 128) return false;
+  static_assert(PairVec<float, 2, EQ_COMOV, 1>::value == VecT<float>::n, "the paired tile of 13 points");
+  const int tiles = (int)(ceil_div(N, TX * VecT<float>::n) * ceil_div(N, TY));
+  const bool one_wave = tiles * (int)ceil_div(N, pick_a_chunk(N, tiles)) <= 148 * 2;  // 128 registers
+  return !(one_wave && step13_chunk<float, EQ_COMOV>(ctx) > 6);  // the coupled equations share a shape
 }
 
 int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, int64_t nsteps, cudaStream_t st) {
@@ -797,7 +811,7 @@ int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, i
   if (ctx->p.flags & CF_FLAG_STAGE_KERNELS)
     return f32 ? rk4_steps_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
-  if (!whole_step_route(ctx))
+  if (!whole_step_route(ctx, nsteps))
     return f32 ? rk4_steps_pairs_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
                : rk4_steps_pairs_t<double>(ctx, d_state, t0, dt, step0, nsteps, st);
   return f32 ? rk4_steps_fused_t<float>(ctx, d_state, t0, dt, step0, nsteps, st)
@@ -809,7 +823,7 @@ int rk4_steps(cf_ctx *ctx, void *d_state, double t0, double dt, int64_t step0, i
 // step in place run on a copy.
 int rk4_step_to(cf_ctx *ctx, const void *from, void *to, double t0, double dt, int64_t step, cudaStream_t st) {
   const bool f32 = ctx->p.precision == CF_FP32_COMP;
-  if (shape_of(ctx->p.equation) == EQ_FRW && whole_step_route(ctx)) {
+  if (shape_of(ctx->p.equation) == EQ_FRW && whole_step_route(ctx, 1)) {
     const double t = t0 + (double)step * dt;
     return f32 ? step_to_t<float>(ctx, from, to, t, dt, st) : step_to_t<double>(ctx, from, to, t, dt, st);
   }
