@@ -388,10 +388,13 @@ static int launch_adj_h(cf_adjoint *adj, const AdjArgs<S> &A, cudaStream_t st) {
   return launch_adj<S, 1, STAGE>(adj, A, st);
 }
 
-// Tiles and planes per CTA of the whole reverse step.
+// Tiles and planes per CTA of the whole reverse step.  A lone CTA's plane takes the same time at 3 CTAs
+// per SM as at 4, 4/3 of a full SM's share (us per reverse step in a sweep of 8 with their forward
+// steps, the chunk without / with it): N = 48 22.9 / 22.8, 56 27.2 / 26.6, 64 28.9 / 26.4, 72 and up the
+// same chunk.
 static dim3 adj_step_grid(long long N, int *a_chunk) {
   const unsigned gx = ceil_div(N, AS_TX * 2), gy = ceil_div(N, AS_TY);
-  *a_chunk = step_a_chunk((int)N, (int)(gx * gy), AS_MB, 4, step_latency(8, false));
+  *a_chunk = step_a_chunk((int)N, (int)(gx * gy), AS_MB, 4, 4.0 / AS_MB * step_latency(8, false));
   return dim3(gx, gy, ceil_div(N, *a_chunk));
 }
 
