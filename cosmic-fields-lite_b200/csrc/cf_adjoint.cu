@@ -60,9 +60,11 @@ struct AdjArgs {
   double two_m;
 };
 
-// STAGE is the forward stage index being reversed: 4, 3, 2 or 1.
-template <typename S, int H, int STAGE>
+// One reverse stage of the 13-point stencil (H = 2 sites wide); STAGE is the forward stage index
+// being reversed: 4, 3, 2 or 1.
+template <typename S, int STAGE>
 __global__ void __launch_bounds__(ATX *ATY) k_adj_stage(const AdjArgs<S> A) {
+  constexpr int H = 2;
   constexpr int TW = ATX * 2;  // two sites per thread (double2)
   constexpr int SP = TW + 2 * H;
   constexpr int SR = ATY + 2 * H;
@@ -145,17 +147,11 @@ __global__ void __launch_bounds__(ATX *ATY) k_adj_stage(const AdjArgs<S> A) {
     for (int v = 0; v < 2; ++v) {
       const int col = H + tx * 2 + v, row = ty + H;
       const double f0 = q[H][v];
-      double lap;
-      if constexpr (H == 1) {
-        lap = -6.0 * f0 + q[2][v] + q[0][v] + sm[(row + 1) * SP + col] + sm[(row - 1) * SP + col] +
-              (sm[row * SP + col + 1] + sm[row * SP + col - 1]);
-      } else {
-        const double s1 = q[3][v] + q[1][v] + sm[(row + 1) * SP + col] + sm[(row - 1) * SP + col] +
-                          sm[row * SP + col + 1] + sm[row * SP + col - 1];
-        const double s2 = q[4][v] + q[0][v] + sm[(row + 2) * SP + col] + sm[(row - 2) * SP + col] +
-                          sm[row * SP + col + 2] + sm[row * SP + col - 2];
-        lap = (16.0 * s1 - s2 - 90.0 * f0) / 12.0;
-      }
+      const double s1 = q[3][v] + q[1][v] + sm[(row + 1) * SP + col] + sm[(row - 1) * SP + col] +
+                        sm[row * SP + col + 1] + sm[row * SP + col - 1];
+      const double s2 = q[4][v] + q[0][v] + sm[(row + 2) * SP + col] + sm[(row - 2) * SP + col] +
+                        sm[row * SP + col + 2] + sm[row * SP + col - 2];
+      const double lap = (16.0 * s1 - s2 - 90.0 * f0) / 12.0;
       const double kv = A.sin * f0, ku = A.sin * uu[v];
       const double ybp = -A.m2 * kv + A.inv * (A.sin * lap);
       const double ybq = ku - A.hub3 * kv;
@@ -351,7 +347,7 @@ struct cf_adjoint {
   bool have_forward = false;
   size_t state_bytes = 0;
   std::vector<void *> ckpt;
-  void *seg = nullptr;  // `every` states
+  void *seg = nullptr;  // a segment's states after its checkpoint
   void *Y = nullptr;    // forward stage inputs y2, y3, y4 (storage type, 2N^3 each)
   double *lam = nullptr, *ka = nullptr, *kb = nullptr, *accb = nullptr, *rb = nullptr;
   double *dm_partial = nullptr;
@@ -369,7 +365,7 @@ static unsigned gridn(long long n, int per = 256) {
   return (unsigned)(b < 1 ? 1 : b);
 }
 
-template <typename S, int H, int STAGE>
+template <typename S, int STAGE>
 static int launch_adj(cf_adjoint *adj, AdjArgs<S> A, cudaStream_t st) {
   cf_ctx *ctx = adj->ctx;
   constexpr int TW = ATX * 2;
@@ -377,15 +373,9 @@ static int launch_adj(cf_adjoint *adj, AdjArgs<S> A, cudaStream_t st) {
   const unsigned gx = ceil_div(A.N, TW), gy = (unsigned)(A.N / ATY);
   A.a_chunk = 16;
   dim3 grid(gx, gy, ceil_div(A.N, A.a_chunk));
-  k_adj_stage<S, H, STAGE><<<grid, block, 0, st>>>(A);
+  k_adj_stage<S, STAGE><<<grid, block, 0, st>>>(A);
   CF_LAUNCHED(ctx);
   return CF_OK;
-}
-
-template <typename S, int STAGE>
-static int launch_adj_h(cf_adjoint *adj, const AdjArgs<S> &A, cudaStream_t st) {
-  if (adj->ctx->p.stencil == 13) return launch_adj<S, 2, STAGE>(adj, A, st);
-  return launch_adj<S, 1, STAGE>(adj, A, st);
 }
 
 // Tiles and planes per CTA of the whole reverse step.  A lone CTA's plane takes the same time at 3 CTAs
@@ -440,21 +430,30 @@ int adjoint_create(cf_ctx *ctx, int64_t nsteps, int64_t every, cf_adjoint **out)
   a->state_bytes = 16 * (size_t)ctx->N3;
   const size_t sb = a->state_bytes, fb = 8 * (size_t)ctx->N3;
   const long long nck = (nsteps + every - 1) / every;
-  auto alloc = [&](void **p, size_t bytes) -> bool { return cudaMalloc(p, bytes) == cudaSuccess; };
+  size_t need = 0;
   bool ok = true;
+  auto alloc = [&](void **p, size_t bytes) {
+    need += bytes;
+    ok = ok && (bytes == 0 || cudaMalloc(p, bytes) == cudaSuccess);
+  };
   a->ckpt.assign(nck, nullptr);
-  for (auto &p : a->ckpt) ok = ok && alloc(&p, sb);
-  ok = ok && alloc(&a->seg, sb * (size_t)every);
-  ok = ok && alloc((void **)&a->lam, 2 * fb) && alloc((void **)&a->ka, 2 * fb) && alloc((void **)&a->rb, fb);
-  if (ctx->p.stencil != 7)  // the single-stage route
-    ok = ok && alloc(&a->Y, 3 * sb) && alloc((void **)&a->kb, 2 * fb) && alloc((void **)&a->accb, 2 * fb);
-  if (ctx->p.stencil == 7) a->grid = adj_step_grid(ctx->N, &a->a_chunk);
+  for (auto &p : a->ckpt) alloc(&p, sb);
+  alloc(&a->seg, sb * (size_t)(every - 1));
+  alloc((void **)&a->lam, 2 * fb);
+  alloc((void **)&a->ka, 2 * fb);
+  alloc((void **)&a->rb, fb);
+  if (ctx->p.stencil == 7) {
+    a->grid = adj_step_grid(ctx->N, &a->a_chunk);
+  } else {  // the single-stage route
+    alloc(&a->Y, 3 * sb);
+    alloc((void **)&a->kb, 2 * fb);
+    alloc((void **)&a->accb, 2 * fb);
+  }
   a->dm_slots = std::max<long long>(adj_cta_count(a), 148 * 16);
-  ok = ok && alloc((void **)&a->dm_partial, sizeof(double) * (size_t)a->dm_slots);
+  alloc((void **)&a->dm_partial, sizeof(double) * (size_t)a->dm_slots);
   if (!ok) {
     cudaGetLastError();
-    set_error("adjoint: device allocation failed (checkpoints + segment need %zu bytes)",
-              sb * (size_t)(nck + every + 3) + 9 * fb);
+    set_error("adjoint: device allocation failed (%zu bytes needed)", need);
     *out = a;
     return CF_ERR_NOMEM;
   }
@@ -578,7 +577,7 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
     const int64_t len = std::min<int64_t>(a->every, a->nsteps - n0);
     char *seg = (char *)a->seg;
     // state j of the segment: the checkpoint itself, then the kept states
-    auto state = [&](int64_t j) { return j == 0 ? (char *)a->ckpt[sgi] : seg + j * sb; };
+    auto state = [&](int64_t j) { return j == 0 ? (char *)a->ckpt[sgi] : seg + (j - 1) * sb; };
     for (int64_t j = 1; j < len; ++j) CF_TRY(rk4_step_to(ctx, state(j - 1), state(j), a->t0, dt, n0 + j - 1, st));
     for (int64_t j = len - 1; j >= 0; --j) {
       const int64_t n = n0 + j;
@@ -615,7 +614,7 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
       A.cl = dt3;
       A.cy = dt;
       A.yphi = Y4;
-      CF_TRY(launch_adj_h<S, 4>(a, A, st));
+      CF_TRY(launch_adj<S, 4>(a, A, st));
       // reverse stage 3 at t + dt/2
       stage_coeffs(ctx->p, t + dh, &inv, &H);
       A.inv = inv;
@@ -626,14 +625,14 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
       A.cl = dt3;
       A.cy = dh;
       A.yphi = Y3;
-      CF_TRY(launch_adj_h<S, 3>(a, A, st));
+      CF_TRY(launch_adj<S, 3>(a, A, st));
       // reverse stage 2 at t + dt/2
       A.kin = a->kb;
       A.knext = a->ka;
       A.cl = dt6;
       A.cy = dh;
       A.yphi = Y2;
-      CF_TRY(launch_adj_h<S, 2>(a, A, st));
+      CF_TRY(launch_adj<S, 2>(a, A, st));
       // reverse stage 1 at t: l = l' + acc + yb1
       stage_coeffs(ctx->p, t, &inv, &H);
       A.inv = inv;
@@ -642,7 +641,7 @@ static int backward_t(cf_adjoint *a, double *d_lambda0, double *h_dm, cudaStream
       A.knext = nullptr;
       A.lam_out = a->lam;
       A.yphi = x;
-      CF_TRY(launch_adj_h<S, 1>(a, A, st));
+      CF_TRY(launch_adj<S, 1>(a, A, st));
     }
   }
   if (d_lambda0)
