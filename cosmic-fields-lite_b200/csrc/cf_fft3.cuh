@@ -28,12 +28,6 @@ __device__ __forceinline__ C64 z_mul(C64 a, C64 b) { return C64{a.x * b.x - a.y 
 __device__ __forceinline__ C64 z_i(C64 a) { return C64{-a.y, a.x}; }  // i a
 
 // v_k = sum_j v_j e^{2 pi i j k / R}, natural order
-__device__ __forceinline__ void bfly(C64 (&)[1]) {}
-__device__ __forceinline__ void bfly(C64 (&v)[2]) {
-  const C64 t = v[0];
-  v[0] = z_add(t, v[1]);
-  v[1] = z_sub(t, v[1]);
-}
 __device__ __forceinline__ void bfly(C64 (&v)[3]) {
   constexpr double h = 0.86602540378443864676;  // sqrt(3)/2
   const C64 t = z_add(v[1], v[2]), d = z_sub(v[1], v[2]);

@@ -31,10 +31,6 @@ namespace cfb {
 template <typename S, int V>
 struct VecOf;
 template <>
-struct VecOf<double, 1> {
-  using T = double;
-};
-template <>
 struct VecOf<double, 2> {
   using T = double2;
 };
@@ -60,9 +56,7 @@ struct Pack {
 template <typename S, int V>
 __device__ __forceinline__ Pack<S, V> unpack(const typename VecOf<S, V>::T &t) {
   Pack<S, V> r;
-  if constexpr (V == 1) {
-    r.v[0] = t;
-  } else if constexpr (V == 2) {
+  if constexpr (V == 2) {
     r.v[0] = t.x;
     r.v[1] = t.y;
   } else {
@@ -89,9 +83,7 @@ __device__ __forceinline__ Pack<S, V> ldv_rw(const S *p) {
 template <typename S, int V>
 __device__ __forceinline__ void stv(S *p, const Pack<S, V> &r) {
   typename VecOf<S, V>::T t;
-  if constexpr (V == 1) {
-    t = r.v[0];
-  } else if constexpr (V == 2) {
+  if constexpr (V == 2) {
     t.x = r.v[0];
     t.y = r.v[1];
   } else {
