@@ -343,8 +343,14 @@ __global__ void __launch_bounds__(256) k_spec_bin(SpecIn A, long long hc_count, 
   }
 }
 
+// (lo, hi) 2^-e, rounded once: the top 64 bits with what is below them in the last one.  (Rounding the
+// two words and their sum, a bin whose high word passes 53 bits carried up to two roundings more.)
 __device__ __forceinline__ double fixed_to_double(unsigned long long lo, unsigned long long hi, int e) {
-  return ldexp(ldexp(__ull2double_rn(hi), 64) + __ull2double_rn(lo), -e);
+  if (hi == 0) return ldexp(__ull2double_rn(lo), -e);
+  const int s = __clzll((long long)hi);
+  unsigned long long top = s ? (hi << s) | (lo >> (64 - s)) : hi;
+  if (lo << s) top |= 1;
+  return ldexp(__ull2double_rn(top), 64 - s - e);
 }
 
 __global__ void k_spec_final(const unsigned long long *bins, const unsigned long long *maxbits, long long pairs,
