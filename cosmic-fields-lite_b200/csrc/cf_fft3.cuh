@@ -66,7 +66,8 @@ __device__ __forceinline__ void bfly(C64 (&v)[8]) {
 }
 
 // Radices of the lengths the passes are built for (R3 = 1: two passes): the column lines N and
-// the packed rows N/2 of the lattices N = 64 ... 1024 of the form 2^k and 3 2^k.
+// the packed rows N/2 of the lattices N = 64 ... 512 of the form 2^k and 3 2^k (fft3_has); others take
+// the transfer kernel, the cuFFT transform and the exponential.
 template <int N>
 struct FftRadix;
 template <> struct FftRadix<32> { static constexpr int R1 = 8, R2 = 4, R3 = 1; };

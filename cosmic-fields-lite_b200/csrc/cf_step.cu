@@ -4,7 +4,8 @@
 // default cf_rk4_steps runs a step as one whole-step pass -- k_step
 // (cf_step_tile.cuh) for the 7-point stencil, k_step13 (cf_step13_tile.cuh) for the
 // 13-point one.  The two paired-stage passes (stages 1+2, 3+4; cf_pair_tile.cuh) remain
-// for CF_FLAG_PAIR_KERNELS and the 13-point batched ensembles; all keep the intermediate
+// for small FP32_COMP 13-point lattices with a curvature input (whole_step_route),
+// CF_FLAG_PAIR_KERNELS and the 13-point batched ensembles; all keep the intermediate
 // stage inputs out of HBM and give the same bits.  The four single-stage kernels remain for
 // CF_FLAG_STAGE_KERNELS, the adjoint's recompute, cf_rk4_steps_noalloc and the
 // 13-point persistent ensemble kernel.  A single-stage kernel makes ONE pass over HBM:
@@ -389,7 +390,7 @@ static int rk4_steps_pairs_t(cf_ctx *ctx, void *d_state, double t0, double dt, i
 //   FP32         32 x 8 threads, 128 x 8 sites (the approximate equation 64 x 8), 2 CTAs/SM.
 //                64 x 16 sites: N = 512 FRW 1.05 against 1.06 ms per step, comoving 2.41 against
 //                2.35, N = 200 FRW 0.114 against 0.109.  128 x 16 at 1 CTA/SM: 1.17.
-//   FP64         16 x 8 threads, 32 x 8 sites at 4 CTAs/SM (102 registers): N = 256 FRW 0.192
+//   FP64         16 x 8 threads, 32 x 8 sites at 4 CTAs/SM (96 registers): N = 256 FRW 0.192
 //                ms against 0.223 at 3 CTAs/SM; 64 x 8 at 2 CTAs/SM 0.216.  The sqrt
 //                potential, whose root needs more registers, 3 CTAs/SM: 0.266 against 0.338.
 //   FP64 comoving 32 x 8 threads, 64 x 8 sites, 2 CTAs/SM: 32 x 8 sites at 4 / 3 CTAs/SM
@@ -851,10 +852,10 @@ struct ScaleSumArgs {
   int n;
 };
 
-// n inputs known (NV) and every array 16-byte aligned: 16-byte vectors, four pieces of each input
-// in flight per thread; the same products and sums in the same order as the general form.
-// What bounds it is HBM: N = 256, two / five inputs 126 / 234 us (6.4 / 6.9 TB/s) against 166 / 244
-// for the general form.
+// n inputs known (NV) and every array 16-byte aligned: 16-byte vectors; the same products and sums in the
+// same order as the general form.  (`out` may be an input, so a thread's pieces follow one another: its
+// loads do not pass its earlier stores.)  What bounds it is HBM: N = 256, two / five inputs 126 / 234 us (6.4 /
+// 6.9 TB/s) against 166 / 244 for the general form.
 template <int NV>
 __global__ void __launch_bounds__(256) k_scale_sum_v(const ScaleSumArgs A) {
   const long long n = A.len / 2;

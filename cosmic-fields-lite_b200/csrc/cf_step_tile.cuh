@@ -51,7 +51,8 @@
 // form the 1-ring's rows and columns of phase 1.  Each role has a loop of its own, so a
 // thread holds the registers of one role only (this, and keeping what one plane leaves for
 // the next in registers or in shared memory by equation, StepKeep, is what fits the
-// register budget without spills), and both meet at one named barrier per plane.
+// register budget: no spills but 4 to 8 bytes for the FP64 lambda phi^4 form and 4 to 24 for the
+// FP64 approximate comoving one), and both meet at one named barrier per plane.
 //
 // What bounds it: latency and shared-memory bandwidth, not HBM -- at N = 256 the FP32 FRW
 // pass issues in 51% of the cycles and the shared-memory pipe is busy in 69% (FP64: 82%).
@@ -121,8 +122,8 @@ constexpr int step_vec() {
 // ya_phi of q - 1; the rest it reads back from shared memory:
 //   x  x_phi, ya_phi of q as well       y  yb_phi, yc_phi of r and r - 1
 //   p  x_pi of q and r (else in shared memory, 3 planes of own sites)
-// FP64 is bound by shared memory, so the uncoupled equations keep all that fits 102 registers
-// (N = 256 FRW: x 0.202 -> 0.201, x and y 0.192 ms; on ragged tiles x and y spill: N = 200
+// FP64 is bound by shared memory, so the uncoupled equations keep all that fits the 96
+// registers of 4 CTAs per SM (N = 256 FRW: x 0.202 -> 0.201, x and y 0.192 ms; on ragged tiles x and y spill: N = 200
 // 0.118 -> 0.155).  The coupled equations hold the curvature of two stages in registers
 // and need the room: FP32 comoving with x_pi in registers 2.70, in shared memory 2.36 ms
 // (N = 512).
@@ -291,7 +292,10 @@ constexpr int step_ring_rows(int TXv, int TYv) {
 
 // The least time of a plane, in the units of step_a_chunk (1.27 on a full SM): a lone CTA's chain of
 // dependent steps.  Measured per plane with one CTA per SM against a full one: FP64 0.76 / 1.66
-// us (5 of 20 warps), FP32 1.19 / 1.59 us, comoving 2.16 / 2.56 us (10 of 20 warps).
+// us (5 of 20 warps), FP32 1.19 / 1.59 us, comoving 2.16 / 2.56 us (10 of 20 warps).  These are of the
+// 7-point pass at 4 (FP64) or 2 CTAs per SM; at fewer a lone CTA has a larger share of a full SM's time
+// (its callers' 4 / CTAs per SM).  In the 13-point pass's 2 or 1 CTAs per SM only the uncoupled FP32
+// value exceeds 0.27 + c / per_sm at c = 1 and acts.
 constexpr double step_latency(size_t word, bool coupled) { return word == 8 ? 0.62 : (coupled ? 1.05 : 0.95); }
 
 __device__ __forceinline__ void step_barrier(int threads) { asm volatile("bar.sync 1, %0;\n" ::"r"(threads) : "memory"); }
