@@ -4,7 +4,7 @@
 // default cf_rk4_steps runs a step as one whole-step pass -- k_step
 // (cf_step_tile.cuh) for the 7-point stencil, k_step13 (cf_step13_tile.cuh) for the
 // 13-point one.  The two paired-stage passes (stages 1+2, 3+4; cf_pair_tile.cuh) remain
-// for small FP32_COMP 13-point lattices with a curvature input (whole_step_route),
+// for some small lattices with a curvature input (whole_step_route),
 // CF_FLAG_PAIR_KERNELS and the 13-point batched ensembles; all keep the intermediate
 // stage inputs out of HBM and give the same bits.  The four single-stage kernels remain for
 // CF_FLAG_STAGE_KERNELS, the adjoint's recompute, cf_rk4_steps_noalloc and the
@@ -785,22 +785,25 @@ int rk4_step_buffers(cf_ctx *ctx, void *d_state, void *acc, void *ya, void *yb, 
   return rk4_step_buffers_t<double>(ctx, d_state, acc, ya, yb, t, dt, st);
 }
 
-// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).  The FP32 13-point
-// pass with a curvature input has one CTA per SM, and the paired passes remain where that costs more
-// than the traffic they add (us per step, whole / paired):
-//   - comoving with the next step's Psi refreshes beside the step (psi_pipelined), which the pass
-//     leaves no room: N = 40 57 / 53, 48 66 / 60, 72 78 / 73, 96 108 / 103, 120 161 / 155.  From N = 128 the pass
-//     gains more than it delays them: 128 85 / 89, 136 238 / 254, 160 223 / 272;
-//   - else, where one wave takes all CTAs of a paired pass, which then march 4 planes, and the whole
-//     pass marches more than 6 (and 8 halo planes): fixed Psi N = 80 (6) 22.6 / 22.7, 88 (8) 26.7 / 23.7,
-//     96 (8) 26.0 / 25.4, 104 (two paired waves) 32.9 / 39.9; one comoving step per call 72 99 / 101,
-//     88 118 / 114, 96 129 / 123, 120 179 / 184; approximate 96 72 / 70.
+// Whether cf_rk4_steps takes whole-step passes (not single-stage or paired ones).  The paired passes, in
+// small CTAs of 256 threads, remain on small lattices where that costs more than the traffic and launch they
+// add (us per step, whole / paired):
+//   - comoving with the next step's Psi refreshes beside the step (psi_pipelined), which large CTAs leave no
+//     room.  From N = 40 to 64 the refreshes are the longer chain: FP64 N = 48 7-point 66 / 62, 13-point 67 /
+//     63, FP32 7-point 59 / 56, N = 64 45 / 43 (at 32 and below launches bound both; N = 72 FP64 82 / 82, 96 130 /
+//     144).  The FP32 13-point pass, alone on its SM, loses up to N = 120: 72 78 / 73, 96 108 / 103, 120 161 /
+//     155, but 128 85 / 89, 136 238 / 254, 160 223 / 272;
+//   - else the FP32 13-point pass with a curvature input, where one wave takes all CTAs of a paired pass,
+//     which then march 4 planes, and the whole pass marches more than 6 (and 8 halo planes): fixed Psi N = 80
+//     (6) 22.6 / 22.7, 88 (8) 26.7 / 23.7, 96 (8) 26.0 / 25.4, 104 (two paired waves) 32.9 / 39.9; one comoving step
+//     per call 72 99 / 101, 88 118 / 114, 96 129 / 123, 120 179 / 184; approximate 96 72 / 70.
 static bool whole_step_route(cf_ctx *ctx, int64_t nsteps) {
   if (ctx->p.flags & (CF_FLAG_STAGE_KERNELS | CF_FLAG_PAIR_KERNELS)) return false;
   const int eq = shape_of(ctx->p.equation), N = (int)ctx->N;
   const bool coupled = eq == EQ_COMOV || eq == EQ_FIXED || eq == EQ_APPROX;
-  if (ctx->p.stencil != 13 || ctx->p.precision != CF_FP32_COMP || !coupled) return true;
-  if (psi_pipelined(ctx, nsteps) && N < 128) return false;
+  const bool alone = ctx->p.stencil == 13 && ctx->p.precision == CF_FP32_COMP && coupled;  // 1 CTA per SM
+  if (psi_pipelined(ctx, nsteps) && N > 32 && (N <= 64 || (alone && N < 128))) return false;
+  if (!alone) return true;
   static_assert(PairVec<float, 2, EQ_COMOV, 1>::value == VecT<float>::n, "the paired tile of 13 points");
   const int tiles = (int)(ceil_div(N, TX * VecT<float>::n) * ceil_div(N, TY));
   const bool one_wave = tiles * (int)ceil_div(N, pick_a_chunk(N, tiles)) <= 148 * 2;  // 128 registers

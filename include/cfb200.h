@@ -110,8 +110,8 @@ typedef struct cf_params {
  * route; every route gives bit-identical states. */
 #define CF_FLAG_STAGE_KERNELS 2
 /* cf_rk4_steps runs each step as two paired-stage passes (stages 1+2, 3+4)
- * instead of one whole-step pass (the default for both stencils; some small FP32_COMP
- * 13-point lattices with a curvature input take the paired passes anyway). */
+ * instead of one whole-step pass (the default for both stencils; some small
+ * lattices with a curvature input take the paired passes anyway). */
 #define CF_FLAG_PAIR_KERNELS 4
 /* FP32 storage: the pruned Psi synthesis's last pass (the length-N C2R of every row)
  * runs as the CTA-per-tile kernel instead of the default warp-per-row-group kernel

@@ -1,5 +1,5 @@
-"""Which passes cf_rk4_steps takes where the choice depends on the lattice and the call (FP32_COMP, 13
-points, a curvature input), and that each route gives the bits of the four single-stage passes, which
+"""Which passes cf_rk4_steps takes where the choice depends on the lattice and the call (a curvature
+input), and that each route gives the bits of the four single-stage passes, which
 share neither tiles nor chunks with them."""
 import numpy as np
 import pytest
@@ -36,19 +36,26 @@ def run(N, eq, prec, flags, nsteps, stencil):
     return out, prof["step"][0], prof["pair_a"][0]
 
 
-# (equation, N, steps, whole-step passes)
-ROUTES = [(FIXED, 72, 2, True), (FIXED, 80, 1, True), (FIXED, 88, 2, False), (FIXED, 96, 1, False), (FIXED, 104, 2, True),
-          (APPROX, 72, 2, True), (APPROX, 96, 2, False), (APPROX, 104, 1, True),
-          (COMOVING, 40, 1, True), (COMOVING, 40, 2, False), (COMOVING, 72, 1, True), (COMOVING, 72, 3, False),
-          (COMOVING, 88, 1, False), (COMOVING, 104, 1, True), (COMOVING, 120, 3, False), (COMOVING, 128, 2, True),
-          (COMOVING, 136, 1, True), (COMOVING, 200, 3, True)]
+FP64, COMP = cfb200.FP64, cfb200.FP32_COMP
+
+# (precision, stencil, equation, N, steps, whole-step passes)
+ROUTES = [(COMP, 13, FIXED, 72, 2, True), (COMP, 13, FIXED, 80, 1, True), (COMP, 13, FIXED, 88, 2, False),
+          (COMP, 13, FIXED, 96, 1, False), (COMP, 13, FIXED, 104, 2, True), (COMP, 13, APPROX, 72, 2, True),
+          (COMP, 13, APPROX, 96, 2, False), (COMP, 13, APPROX, 104, 1, True), (COMP, 13, COMOVING, 72, 1, True),
+          (COMP, 13, COMOVING, 72, 3, False), (COMP, 13, COMOVING, 88, 1, False), (COMP, 13, COMOVING, 104, 1, True),
+          (COMP, 13, COMOVING, 120, 3, False), (COMP, 13, COMOVING, 128, 2, True), (COMP, 13, COMOVING, 136, 1, True),
+          (COMP, 13, COMOVING, 200, 3, True)]
+ROUTES += [(p, s, COMOVING, N, n, whole) for p in (FP64, COMP) for s in (7, 13)
+           for N, n, whole in ((32, 2, True), (40, 1, True), (40, 2, False), (64, 3, False))]
+ROUTES += [(FP64, 13, FIXED, 88, 2, True), (FP64, 7, COMOVING, 72, 2, True), (FP64, 13, COMOVING, 72, 2, True),
+           (COMP, 7, COMOVING, 72, 2, True)]
 
 
-@pytest.mark.parametrize("eq,N,nsteps,whole", ROUTES)
-def test_route_and_bits(eq, N, nsteps, whole):
-    out, step, pair = run(N, eq, cfb200.FP32_COMP, 0, nsteps, 13)
+@pytest.mark.parametrize("prec,stencil,eq,N,nsteps,whole", ROUTES)
+def test_route_and_bits(prec, stencil, eq, N, nsteps, whole):
+    out, step, pair = run(N, eq, prec, 0, nsteps, stencil)
     assert (step, pair) == ((nsteps, 0) if whole else (0, nsteps))
-    want, step, pair = run(N, eq, cfb200.FP32_COMP, cfb200.FLAG_STAGE_KERNELS, nsteps, 13)
+    want, step, pair = run(N, eq, prec, cfb200.FLAG_STAGE_KERNELS, nsteps, stencil)
     assert (step, pair) == (0, 0)
     assert torch.equal(out, want)
 
