@@ -438,30 +438,38 @@ static unsigned grid_for(long long n, int per = 256) {
   return (unsigned)b;
 }
 
-int ensure_spectrum_scratch(cf_ctx *ctx, int nfields) {
-  const size_t hc = (size_t)ctx->hc_count;
-  if (!ctx->spec_hc) {
-    if (cudaMalloc(&ctx->spec_hc, 2 * hc * sizeof(double)) != cudaSuccess) {
-      set_error("cudaMalloc spectrum HC scratch failed");
-      return CF_ERR_NOMEM;
-    }
-    if (cudaMalloc(&ctx->spec_field, 2 * (size_t)ctx->N3 * sizeof(double)) != cudaSuccess) {
-      set_error("cudaMalloc spectrum field scratch failed");
-      return CF_ERR_NOMEM;
-    }
-    if (cudaMalloc(&ctx->bins, 2 * (size_t)ctx->s2_bins * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&ctx->maxbits, 2 * sizeof(unsigned long long)) != cudaSuccess ||
-        cudaMalloc(&ctx->s2_counts, (size_t)ctx->s2_bins * sizeof(int64_t)) != cudaSuccess) {
-      set_error("cudaMalloc spectrum bins failed");
-      return CF_ERR_NOMEM;
-    }
-    CF_TRY_CUDA(cudaMemset(ctx->s2_counts, 0, (size_t)ctx->s2_bins * sizeof(int64_t)));
-    k_s2_counts<<<orbit_blocks((int)ctx->N), 256>>>((int)ctx->N, (unsigned long long *)ctx->s2_counts);
-    CF_LAUNCHED(ctx);
-    CF_TRY_CUDA(cudaMemset(ctx->bins, 0, 2 * (size_t)ctx->s2_bins * sizeof(unsigned long long)));
-    CF_TRY_CUDA(cudaMemset(ctx->maxbits, 0, 2 * sizeof(unsigned long long)));
-    CF_TRY_CUDA(cudaDeviceSynchronize());
+// The scratch of the spectra, all of it or none: a later call takes spec_hc for the sign that it is there.
+static int alloc_spectrum_scratch(cf_ctx *ctx) {
+  const size_t hc = (size_t)ctx->hc_count, nb = (size_t)ctx->s2_bins;
+  void *p[5] = {};
+  const size_t bytes[5] = {2 * hc * sizeof(double), 2 * (size_t)ctx->N3 * sizeof(double),
+                           2 * nb * sizeof(unsigned long long), 2 * sizeof(unsigned long long), nb * sizeof(int64_t)};
+  cudaError_t e = cudaSuccess;
+  for (int k = 0; k < 5 && e == cudaSuccess; ++k) e = cudaMalloc(&p[k], bytes[k]);
+  const bool nomem = e != cudaSuccess;
+  for (int k = 2; k < 5 && e == cudaSuccess; ++k) e = cudaMemset(p[k], 0, bytes[k]);
+  if (e == cudaSuccess) {
+    k_s2_counts<<<orbit_blocks((int)ctx->N), 256>>>((int)ctx->N, (unsigned long long *)p[4]);
+    ctx->launches++;
+    e = cudaGetLastError();
   }
+  if (e == cudaSuccess) e = cudaDeviceSynchronize();
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    for (void *q : p) cudaFree(q);
+    set_error("spectrum scratch (%zu bytes): %s", bytes[0] + bytes[1] + bytes[2] + bytes[3] + bytes[4], cudaGetErrorString(e));
+    return nomem ? CF_ERR_NOMEM : CF_ERR_CUDA;
+  }
+  ctx->spec_hc = (double *)p[0];
+  ctx->spec_field = (double *)p[1];
+  ctx->bins = (unsigned long long *)p[2];
+  ctx->maxbits = (unsigned long long *)p[3];
+  ctx->s2_counts = (int64_t *)p[4];
+  return CF_OK;
+}
+
+int ensure_spectrum_scratch(cf_ctx *ctx, int nfields) {
+  if (!ctx->spec_hc) CF_TRY(alloc_spectrum_scratch(ctx));
   const int N = (int)ctx->N;
   if (nfields >= 1 && !ctx->have_d2z1) {
     CF_TRY_CUFFT(cufftPlan3d(&ctx->plan_d2z1, N, N, N, CUFFT_D2Z));
@@ -671,8 +679,8 @@ int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, 
   o.mean = d_avg;
   if (!d_slice && !d_avg) return CF_OK;
   if (!d_avg || slices_in_one_march(ctx)) return energy_density_b(ctx, d_state, t, o, st);
-  const long long NN = ctx->N * ctx->N;
   CF_TRY(ensure_spectrum_scratch(ctx, 1));
+  const long long NN = ctx->N * ctx->N;
   CF_TRY(energy_density(ctx, d_state, t, ctx->spec_field, st));
   if (d_slice)
     CF_TRY_CUDA(cudaMemcpyAsync(d_slice, ctx->spec_field, NN * sizeof(double), cudaMemcpyDeviceToDevice, st));
