@@ -678,8 +678,11 @@ int density_slices(cf_ctx *ctx, const void *d_state, double t, double *d_slice, 
   o.slice = d_slice;
   o.mean = d_avg;
   if (!d_slice && !d_avg) return CF_OK;
-  if (!d_avg || slices_in_one_march(ctx)) return energy_density_b(ctx, d_state, t, o, st);
-  CF_TRY(ensure_spectrum_scratch(ctx, 1));
+  const bool march = !d_avg || slices_in_one_march(ctx);
+  const int scratch = march ? CF_OK : ensure_spectrum_scratch(ctx, 0);
+  // without room for the density the march, which needs none, serves every lattice
+  if (march || scratch == CF_ERR_NOMEM) return energy_density_b(ctx, d_state, t, o, st);
+  CF_TRY(scratch);
   const long long NN = ctx->N * ctx->N;
   CF_TRY(energy_density(ctx, d_state, t, ctx->spec_field, st));
   if (d_slice)
