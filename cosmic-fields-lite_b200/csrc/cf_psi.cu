@@ -1426,17 +1426,19 @@ static int alloc_psi_slots(cf_ctx *ctx, int n) {
 }
 
 int ensure_psi(cf_ctx *ctx) {
-  if (ctx->psi_table) return CF_OK;  // buffers in place
+  if (ctx->psi_table) return alloc_psi_slots(ctx, 3);  // in place but for slots that an earlier call found no room for
   const size_t w = ctx->word;
   const size_t hc_bytes = (size_t)ctx->hc_count * w;
   if (!ctx->R_fft) {
     if (cudaMalloc(&ctx->R_fft, hc_bytes) != cudaSuccess) {
+      cudaGetLastError();
       set_error("cudaMalloc R_fft (%zu bytes) failed", hc_bytes);
       return CF_ERR_NOMEM;
     }
     CF_TRY_CUDA(cudaMemset(ctx->R_fft, 0, hc_bytes));
   }
   if (cudaMalloc(&ctx->psi_table, 2 * (size_t)ctx->s2_bins * sizeof(double)) != cudaSuccess) {
+    cudaGetLastError();
     set_error("cudaMalloc transfer table failed");
     return CF_ERR_NOMEM;
   }
