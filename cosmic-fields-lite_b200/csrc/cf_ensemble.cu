@@ -900,8 +900,34 @@ static int segment(cf_ensemble *E, int mode, long long steps, double dt, cudaStr
   return CF_OK;
 }
 
-static int ensure_spectra(cf_ensemble *E) {
-  if (!E->classes.empty()) return CF_OK;
+static void free_classes(std::vector<cf_ensemble::Cls> &classes) {
+  for (auto &c : classes) {
+    cudaFree(c.d_members);
+    cudaFree(c.rho);
+    cudaFree(c.hc);
+    if (c.have_plan) cufftDestroy(c.plan);
+  }
+  classes.clear();
+}
+
+// One size class: its members' densities, half-complex fields and batched transform.
+static int make_class(cf_ensemble::Cls &c, const std::vector<int> &members, long long N) {
+  c.N = (int)N;
+  c.members = members;
+  const long long n = (long long)c.members.size(), N3 = N * N * N, hc = 2 * N * N * (N / 2 + 1);
+  CF_TRY_CUDA(cudaMalloc(&c.d_members, sizeof(int) * n));
+  CF_TRY_CUDA(cudaMemcpy(c.d_members, c.members.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+  CF_TRY_CUDA(cudaMalloc(&c.rho, sizeof(double) * N3 * n));
+  CF_TRY_CUDA(cudaMalloc(&c.hc, sizeof(double) * hc * n));
+  long long nn[3] = {N, N, N}, ie[3] = {N, N, N}, oe[3] = {N, N, N / 2 + 1};
+  size_t work = 0;
+  CF_TRY_CUFFT(cufftCreate(&c.plan));
+  c.have_plan = true;
+  CF_TRY_CUFFT(cufftMakePlanMany64(c.plan, 3, nn, ie, 1, N3, oe, 1, hc / 2, CUFFT_D2Z, n, &work));
+  return CF_OK;
+}
+
+static int make_spectra(cf_ensemble *E, std::vector<cf_ensemble::Cls> &classes) {
   std::map<int, std::vector<int>> byN;
   for (int i = 0; i < E->count; ++i) byN[E->hm[i].N].push_back(i);
   E->out_offset.assign(E->count, 0);
@@ -912,26 +938,30 @@ static int ensure_spectra(cf_ensemble *E) {
     off += 3 * (N / 2) * (N / 2) + 1;
   }
   E->out_total = off;
+  long long bins = 0;
   for (auto &kv : byN) {
-    cf_ensemble::Cls c;
-    c.N = kv.first;
-    c.members = kv.second;
-    const long long N = c.N, n = (long long)c.members.size();
-    const long long N3 = N * N * N, hc = 2 * N * N * (N / 2 + 1);
-    CF_TRY_CUDA(cudaMalloc(&c.d_members, sizeof(int) * n));
-    CF_TRY_CUDA(cudaMemcpy(c.d_members, c.members.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    CF_TRY_CUDA(cudaMalloc(&c.rho, sizeof(double) * N3 * n));
-    CF_TRY_CUDA(cudaMalloc(&c.hc, sizeof(double) * hc * n));
-    long long nn[3] = {N, N, N}, ie[3] = {N, N, N}, oe[3] = {N, N, N / 2 + 1};
-    size_t work = 0;
-    CF_TRY_CUFFT(cufftCreate(&c.plan));
-    CF_TRY_CUFFT(cufftMakePlanMany64(c.plan, 3, nn, ie, 1, N3, oe, 1, hc / 2, CUFFT_D2Z, n, &work));
-    c.have_plan = true;
-    E->max_bins = std::max<long long>(E->max_bins, (3 * (N / 2) * (N / 2) + 1) * n);
-    E->classes.push_back(c);
+    classes.emplace_back();
+    CF_TRY(make_class(classes.back(), kv.second, kv.first));
+    const long long N = kv.first;
+    bins = std::max<long long>(bins, (3 * (N / 2) * (N / 2) + 1) * (long long)kv.second.size());
   }
-  CF_TRY_CUDA(cudaMalloc(&E->d_max, sizeof(unsigned long long) * E->count));
-  CF_TRY_CUDA(cudaMalloc(&E->d_bins, sizeof(unsigned long long) * 2 * E->max_bins));
+  if (!E->d_max) CF_TRY_CUDA(cudaMalloc(&E->d_max, sizeof(unsigned long long) * E->count));
+  if (!E->d_bins) CF_TRY_CUDA(cudaMalloc(&E->d_bins, sizeof(unsigned long long) * 2 * bins));
+  E->max_bins = bins;
+  return CF_OK;
+}
+
+// All of the spectra's buffers or none: a later call takes the classes for the sign that they are there.
+static int ensure_spectra(cf_ensemble *E) {
+  if (!E->classes.empty()) return CF_OK;
+  std::vector<cf_ensemble::Cls> classes;
+  const int s = make_spectra(E, classes);
+  if (s != CF_OK) {
+    cudaGetLastError();
+    free_classes(classes);
+    return s;
+  }
+  E->classes.swap(classes);
   return CF_OK;
 }
 
@@ -1065,12 +1095,7 @@ int cf_ensemble_destroy(cf_ensemble *E) {
   cudaFree(E->d_step);
   cudaFree(E->d_bar);
   cudaFree(E->d_err);
-  for (auto &c : E->classes) {
-    cudaFree(c.d_members);
-    cudaFree(c.rho);
-    cudaFree(c.hc);
-    if (c.have_plan) cufftDestroy(c.plan);
-  }
+  free_classes(E->classes);
   cudaFree(E->d_max);
   cudaFree(E->d_bins);
   delete E;
